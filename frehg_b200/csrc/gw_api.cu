@@ -230,7 +230,7 @@ int frehg_gw_create(const frehg_gw_desc* desc, frehg_gw_handle** out) {
       if (e == cudaSuccess)
         e = dalloc(D, &D.partial, static_cast<size_t>(fgw::kPSlots) * D.nblk);
       if (e == cudaSuccess)
-        e = dalloc(D, &D.cgpart, 4 * static_cast<size_t>(std::max(D.cg_grid, D.cg_grid32)));
+        e = dalloc(D, &D.cgpart, fgw::kSolveSlots * static_cast<size_t>(std::max(D.cg_grid, D.cg_grid32)));
       if (e == cudaSuccess) e = dalloc(D, &D.out, 1);
       return e;
     };

@@ -52,16 +52,23 @@ namespace fgw {
 
 namespace {
 
-// Before a group's solve launch, one block: ranks the members by estimated
+// Before a group's solve launch, block 0: ranks the members by estimated
 // work, nb (iterations of the previous solve + 4), largest first, ties by
 // table index (up to kRankMax members; beyond, table order), writes the queue
 // order and its slot offsets, then zeroes the members' CG states and the
-// slot counter.  The order only decides which member's slots go out first;
+// slot counter; the other blocks zero the members' reduction slots.  The order only decides which member's slots go out first;
 // a member's arithmetic depends on its own block count alone.
 constexpr int kRankMax = 1024;
 
-__global__ void k_queue_setup(CgState** st, const int* __restrict__ first, int n, int* queue,
-                              int* order, int* ofirst) {
+__global__ void k_queue_setup(CgState** st, double* const* __restrict__ parts,
+                              const int* __restrict__ first, int n, int* queue, int* order,
+                              int* ofirst) {
+  if (blockIdx.x > 0) {
+    for (int i = blockIdx.x - 1; i < n; i += gridDim.x - 1)
+      for (int w = threadIdx.x; w < coop::kRedSlots * (first[i + 1] - first[i]); w += blockDim.x)
+        parts[i][w] = 0.0;
+    return;
+  }
   __shared__ int part[256];
   const int t = threadIdx.x;
   if (n <= kRankMax) {
@@ -110,8 +117,7 @@ __global__ void k_queue_setup(CgState** st, const int* __restrict__ first, int n
     s->reason = 0;
     s->outer = 0;
     s->err = 0;
-    s->bar_count = 0u;
-    s->bar_gen = 0u;
+    s->arrived = 0u;
   }
   if (t == 0) *queue = 0;
 }
@@ -142,16 +148,17 @@ int solve_blocks_per_sm(const SolveClass& c, size_t smem) {
 }
 
 int solve_max_blocks(const Device& D, const SolveClass& c) {
-  // The member's reduction buffer holds 4 max(cg_grid, cg_grid32) doubles;
-  // a solve on G blocks uses 3 G of them (FP64) or 4 G (mixed).
-  const int cap = (4 * std::max(D.cg_grid, D.cg_grid32)) / (c.kind == 1 ? 4 : 3);
+  // The member's reduction buffer holds kRedSlots max(cg_grid, cg_grid32)
+  // doubles, kRedSlots a block.
+  (void)c;
+  const int cap = std::max(D.cg_grid, D.cg_grid32);
   return std::max(1, cap);
 }
 
 size_t solve_group_bytes(const SolveClass& c, int n) {
   auto r = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
   return r(args_bytes(c) * n) + r(sizeof(int) * (n + 1)) + r(sizeof(CgState*) * n) +
-         r(sizeof(int)) + r(sizeof(int) * n) + r(sizeof(int) * (n + 1));
+         r(sizeof(double*) * n) + r(sizeof(int)) + r(sizeof(int) * n) + r(sizeof(int) * (n + 1));
 }
 
 cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vector<Device*>& ds,
@@ -163,12 +170,14 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   std::vector<unsigned char> tab(ab * ds.size());
   std::vector<int> first(ds.size() + 1, 0);
   std::vector<CgState*> st(ds.size());
+  std::vector<double*> parts(ds.size());
   g.smem = 0;
   for (size_t i = 0; i < ds.size(); ++i) {
     if (c.kind == 0) cg64_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
     else mixed_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
     first[i + 1] = first[i] + nb[i];
     st[i] = &ds[i]->out->cg;
+    parts[i] = ds[i]->cgpart;
     if (c.kind == 1) g.smem = std::max(g.smem, mixed_batch_smem(*ds[i], variants[i]));
   }
   g.slots = first.back();
@@ -180,6 +189,8 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   g.states = reinterpret_cast<CgState**>(base + r(tab.size()) + r(first.size() * sizeof(int)));
   char* q = base + r(tab.size()) + r(first.size() * sizeof(int)) +
             r(st.size() * sizeof(CgState*));
+  g.parts = reinterpret_cast<double**>(q);
+  q += r(parts.size() * sizeof(double*));
   g.queue = reinterpret_cast<int*>(q);
   g.order = reinterpret_cast<int*>(q + r(sizeof(int)));
   g.ofirst = reinterpret_cast<int*>(q + r(sizeof(int)) + r(sizeof(int) * ds.size()));
@@ -188,13 +199,15 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
     e = cudaMemcpy(g.first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(g.states, st.data(), st.size() * sizeof(CgState*), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(g.parts, parts.data(), parts.size() * sizeof(double*), cudaMemcpyHostToDevice);
   if (e == cudaSuccess && g.smem > 0)
     e = raise_smem_limit(batch_kernel(c), g.smem);
   return e;
 }
 
 cudaError_t solve_group_launch(const SolveGroup& g, cudaStream_t s) {
-  k_queue_setup<<<1, 256, 0, s>>>(g.states, g.first, g.n, g.queue, g.order, g.ofirst);
+  k_queue_setup<<<1 + std::min(g.n, 128), 256, 0, s>>>(g.states, g.parts, g.first, g.n, g.queue, g.order, g.ofirst);
   void* tab = g.tab;
   int* first = g.first;
   int n = g.n;

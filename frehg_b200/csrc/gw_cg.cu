@@ -11,9 +11,9 @@
 // One persistent cooperative launch runs the whole solve.  Per iteration:
 //   phase A: p_new = z + b p_old (for the seven stencil points), w = A p_new,
 //            partial p'w;
-//   grid barrier; every block reduces the partials in block order;
+//   grid barrier that sums the partials (grid_sum);
 //   phase B: x += a p, r -= a w, z = r / diag, partials z'z and z'r;
-//   grid barrier; reduction; convergence test.
+//   the same barrier; convergence test.
 // Every thread takes two consecutive cells (cg64v_body), with 16-byte pair
 // loads where nz is even and separate loads where it is odd.
 // Per cell and iteration this moves 16 FP64 words (128 B) through HBM:
@@ -22,10 +22,9 @@
 // by L1/L2 because the grid-stride sweep keeps all resident blocks inside a
 // few j-rows of each other.
 //
-// The grid barrier is a bounded spin on a generation counter: a wait that
-// exceeds kSpinLimit polls sets CgState::err, and every block leaves at its
-// next barrier, so a launch that lost co-residency ends with an error status
-// instead of hanging.
+// The grid barrier's wait is bounded: one that exceeds kSpinLimit polls sets
+// CgState::err, and every block leaves at its next barrier, so a launch that
+// lost co-residency ends with an error status instead of hanging.
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -43,7 +42,7 @@ struct Cg64Args {
   Dims d;
   const double *diag, *gxp, *gyp, *gzp, *b;
   double *x, *r, *z, *p0, *p1, *w;
-  double* part;  // 3 x G
+  double* part;  // kRedSlots x G, zero before the launch
   CgState* st;
   double rtol, atol;
   int maxit;
@@ -140,9 +139,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   const long long ct = a.d.ncell - 1;
   const long long stride = static_cast<long long>(G) * blockDim.x;
   const long long t0 = bid * static_cast<long long>(blockDim.x) + threadIdx.x;
-  double* const pzz = a.part;
-  double* const pzr = a.part + G;
-  double* const ppw = a.part + 2 * G;
+  unsigned epoch = 0;
 
   double zz = 0.0, zr = 0.0;
   for (long long q = t0; q < N2; q += stride) {
@@ -161,13 +158,10 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     zr += z1 * rc.y;
   }
   if (tail) cg64_cell_init(a, ct, zz, zr);
-  double s = block_sum_all(zz);
-  if (threadIdx.x == 0) pzz[bid] = s;
-  s = block_sum_all(zr);
-  if (threadIdx.x == 0) pzr[bid] = s;
-  if (!grid_sync(a.st, G)) return;
-  double dp = sqrt(reduce_partials(pzz, G));
-  double beta = reduce_partials(pzr, G);
+  double s2[2] = {zz, zr};
+  if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+  double dp = sqrt(s2[0]);
+  double beta = s2[1];
   const double rnorm0 = dp;
   const double ttol = fmax(a.rtol * rnorm0, a.atol);
   int reason = 0, its = 0;
@@ -233,11 +227,10 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       pw += P1 * w1;
     }
     if (tail) cg64_cell_stencil(a, ct, bc, pold, pnew, pw);
-    s = block_sum_all(pw);
-    if (threadIdx.x == 0) ppw[bid] = s;
-    if (!grid_sync(a.st, G)) return;
+    double s1[1] = {pw};
+    if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
     dpiold = dpi;
-    dpi = reduce_partials(ppw, G);
+    dpi = s1[0];
     betaold = beta;
     if (dpi == 0.0 || (i > 0 && sgn(dpi) * sgn(dpiold) < 0)) {
       reason = -10;
@@ -261,15 +254,13 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       zr += z1 * r1;
     }
     if (tail) cg64_cell_update(a, ct, al, pnew, zz, zr);
-    s = block_sum_all(zz);
-    if (threadIdx.x == 0) pzz[bid] = s;
-    s = block_sum_all(zr);
-    if (threadIdx.x == 0) pzr[bid] = s;
-    if (!grid_sync(a.st, G)) return;
-    dp = sqrt(reduce_partials(pzz, G));
+    s2[0] = zz;
+    s2[1] = zr;
+    if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+    dp = sqrt(s2[0]);
     test(dp);
     if (reason != 0) break;
-    beta = reduce_partials(pzr, G);
+    beta = s2[1];
     ++i;
     if (i >= a.maxit) {
       reason = -3;
@@ -285,13 +276,13 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   }
 }
 
-// Two blocks per SM: at three the 80-register cap spilled (24 bytes a thread)
-// and the 512x512x128 FP64 solve took 251 ms against 236.
-__global__ void __launch_bounds__(kCgBlock, 2) k_cg64v(Cg64Args a) {
+// 128 registers a thread: at an 80-register cap (768 threads per SM) the
+// kernel spilled and the 512x512x128 FP64 solve took 251 ms against 236.
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg64v(Cg64Args a) {
   cg64v_body<true>(a, blockIdx.x, gridDim.x);
 }
 
-__global__ void __launch_bounds__(kCgBlock, 2) k_cg64u(Cg64Args a) {
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg64u(Cg64Args a) {
   cg64v_body<false>(a, blockIdx.x, gridDim.x);
 }
 
@@ -303,7 +294,7 @@ __global__ void __launch_bounds__(kCgBlock, 2) k_cg64u(Cg64Args a) {
 // block whose instance has converged goes on to a waiting instance.  The
 // slot's index within its instance, not the block, fixes the block's share
 // of the instance's cells.
-__global__ void __launch_bounds__(kCgBlock, 3)
+__global__ void __launch_bounds__(kCgBlock, 1)
     k_cg64_batch(const Cg64Args* __restrict__ tab, const int* __restrict__ first, int n,
                  int* queue, const int* __restrict__ order, const int* __restrict__ ofirst) {
   __shared__ Cg64Args sa;
@@ -373,6 +364,7 @@ Cg64Args make_cg64_args(const Device& D, double rtol, double atol, int maxit) {
 
 cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit) {
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * D.cg_grid, D.stream);
   Cg64Args a = make_cg64_args(D, rtol, atol, maxit);
   void* args[] = {&a};
   ++D.launches;

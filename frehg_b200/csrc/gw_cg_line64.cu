@@ -32,7 +32,7 @@ struct Line64Args {
   double *x0, *x1;              // iterate ping-pong (x0 holds h^n at entry)
   const double *dinv, *l;       // column LDL^T factors
   double *r, *z, *p0, *p1, *w, *dd;
-  double* part;                 // 4 x G
+  double* part;                 // kRedSlots x G, zero before the launch
   CgState* st;
   double outer_rtol, inner_rtol, atol;
   int max_inner, max_outer, max_total;
@@ -99,10 +99,7 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
   const bool vec = (nz % E == 0);
   const long long gwarp = bid * static_cast<long long>(kCgBlock / 32) + (threadIdx.x >> 5);
   const long long nwarp = static_cast<long long>(G) * (kCgBlock / 32);
-  double* const q0 = a.part;
-  double* const q1 = a.part + G;
-  double* const q2 = a.part + 2 * G;
-  double* const q3 = a.part + 3 * G;
+  unsigned epoch = 0;
 
   // ||b|| (the first residual is b - A h^n, not b) and d = 0.
   double bb = 0.0;
@@ -111,9 +108,9 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
     bb += bv * bv;
     a.dd[c] = 0.0;
   }
-  double s0 = block_sum_all(bb);
-  if (threadIdx.x == 0) q3[bid] = s0;
-  if (!grid_sync(a.st, G)) return;
+  double s1[1] = {bb};
+  if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
+  bb = s1[0];
 
   double bnorm = 0.0, rnorm = 0.0;
   int total = 0, outer = 0, reason = 0, final_buf = 0;
@@ -164,18 +161,13 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
       st_col<E>(a.r, cb, lane, nz, vec, rv);
       st_col<E>(a.z, cb, lane, nz, vec, zv);
     }
-    double s = block_sum_all(rn2);
-    if (threadIdx.x == 0) q0[bid] = s;
-    s = block_sum_all(zz);
-    if (threadIdx.x == 0) q1[bid] = s;
-    s = block_sum_all(zr);
-    if (threadIdx.x == 0) q2[bid] = s;
-    if (!grid_sync(a.st, G)) return;
-    rnorm = sqrt(reduce_partials(q0, G));
-    const double zn0 = sqrt(reduce_partials(q1, G));
-    double beta = reduce_partials(q2, G);
+    double s3[3] = {rn2, zz, zr};
+    if (!grid_sum(s3, a.part, bid, G, epoch, a.st)) return;
+    rnorm = sqrt(s3[0]);
+    const double zn0 = sqrt(s3[1]);
+    double beta = s3[2];
     final_buf = (o & 1) ? 0 : 1;
-    if (o == 0) bnorm = sqrt(reduce_partials(q3, G));
+    if (o == 0) bnorm = sqrt(bb);
     if (!isfinite(rnorm)) {
       reason = -9;
       break;
@@ -202,10 +194,9 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
       double* __restrict__ pnew = (i & 1) ? a.p0 : a.p1;
       const double pw = (i == 0) ? line64_phase_a<true>(a, bc, pold, pnew, 0.0, t0, stride)
                                  : line64_phase_a<false>(a, bc, pold, pnew, s_pal, t0, stride);
-      s = block_sum_all(pw);
-      if (threadIdx.x == 0) q0[bid] = s;
-      if (!grid_sync(a.st, G)) return;
-      const double dpi = reduce_partials(q0, G);
+      s1[0] = pw;
+      if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
+      const double dpi = s1[0];
       if (!(dpi > 0.0)) break;  // breakdown: keep d, the outer sweep decides
       const double al = beta / dpi;
       betaold = beta;
@@ -237,14 +228,11 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
           }
         }
       }
-      s = block_sum_all(zz);
-      if (threadIdx.x == 0) q1[bid] = s;
-      s = block_sum_all(zr);
-      if (threadIdx.x == 0) q2[bid] = s;
-      if (!grid_sync(a.st, G)) return;
-      const double zn = sqrt(reduce_partials(q1, G));
+      double s2[2] = {zz, zr};
+      if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+      const double zn = sqrt(s2[0]);
       if (zn <= itol) break;
-      beta = reduce_partials(q2, G);
+      beta = s2[1];
     }
   }
   // The solution of the last outer pass lives in x1 after even passes.
@@ -261,7 +249,7 @@ __device__ __forceinline__ void line64_body(const Line64Args& a, const int bid, 
 }
 
 template <int E>
-__global__ void __launch_bounds__(kCgBlock, 2) k_cg_line64(Line64Args a) {
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg_line64(Line64Args a) {
   line64_body<E>(a, blockIdx.x, gridDim.x);
 }
 
@@ -319,10 +307,11 @@ cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rto
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(k),
                                                 kCgBlock, 0);
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  // 4 x g reduction partials fit the 4 x (4 sm_count) doubles allocated at create.
+  // the reduction slots allocated at create serve up to 4 sm_count blocks
   if (per_sm > 4) per_sm = 4;
   const long long g = static_cast<long long>(per_sm) * D.sm_count;
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * g, D.stream);
   Line64Args a;
   a.d = D.d;
   a.diag = D.diag;

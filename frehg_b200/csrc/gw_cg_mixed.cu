@@ -168,7 +168,7 @@ struct MixedArgs {
   double *x0, *x1;
   const float *diag32, *gxp32, *gyp32, *gzp32, *dinv32, *l32;
   float *r32, *z32, *p0, *p1, *w32, *d32;
-  double* part;  // 4 x G
+  double* part;  // kRedSlots x G, zero before the launch
   CgState* st;
   double outer_rtol, inner_rtol, atol;
   int max_inner, max_outer, max_total;
@@ -322,10 +322,7 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
   const bool vec = (E > 0) && (nz % (E > 0 ? E : 1) == 0);
   const long long gwarp = bid * static_cast<long long>(kCgBlock / 32) + (threadIdx.x >> 5);
   const long long nwarp = static_cast<long long>(G) * (kCgBlock / 32);
-  double* const q0 = a.part;
-  double* const q1 = a.part + G;
-  double* const q2 = a.part + 2 * G;
-  double* const q3 = a.part + 3 * G;
+  unsigned epoch = 0;
 
   // A warm start begins from the assembly's x0 = h^n; the outer test is
   // relative to ||b||, reduced here since the first residual is no longer b.
@@ -339,18 +336,14 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
     }
     a.d32[c] = 0.0f;
   }
-  if (a.warm) {
-    const double s0 = block_sum_all(bb);
-    if (threadIdx.x == 0) q3[bid] = s0;
-  }
-  if (!grid_sync(a.st, G)) return;
+  double s1[1] = {bb};
+  if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
+  bb = s1[0];
 
   double bnorm = 0.0, rnorm = 0.0;
   int total = 0, outer = 0, reason = 0, final_buf = 0;
   // The last inner iteration's update d += s_pal * p_(s_pbuf), applied by
-  // the next phase A or outer pass (s_pal = 0: none).  Shared rather than
-  // loop-carried registers: those spilled the 80-register budget of three
-  // blocks per SM.  Thread 0 writes them only after a grid sync that follows
+  // the next phase A or outer pass (s_pal = 0: none).  Thread 0 writes them only after a grid sync that follows
   // every read of the old values; the next reads follow another grid sync.
   __shared__ float s_pal;
   __shared__ int s_pbuf;
@@ -432,18 +425,13 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
       __syncthreads();
     }
     }
-    double s = block_sum_all(rn2);
-    if (threadIdx.x == 0) q0[bid] = s;
-    s = block_sum_all(zz);
-    if (threadIdx.x == 0) q1[bid] = s;
-    s = block_sum_all(zr);
-    if (threadIdx.x == 0) q2[bid] = s;
-    if (!grid_sync(a.st, G)) return;
-    rnorm = sqrt(reduce_partials(q0, G));
-    const double zn0 = sqrt(reduce_partials(q1, G));
-    double beta = reduce_partials(q2, G);
+    double s3[3] = {rn2, zz, zr};
+    if (!grid_sum(s3, a.part, bid, G, epoch, a.st)) return;
+    rnorm = sqrt(s3[0]);
+    const double zn0 = sqrt(s3[1]);
+    double beta = s3[2];
     final_buf = (o & 1) ? 0 : 1;
-    if (o == 0) bnorm = a.warm ? sqrt(reduce_partials(q3, G)) : rnorm;
+    if (o == 0) bnorm = a.warm ? sqrt(bb) : rnorm;
     if (!isfinite(rnorm)) {
       reason = -9;
       break;
@@ -474,10 +462,9 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
       float* __restrict__ pnew = (i & 1) ? a.p0 : a.p1;
       const double pw = (i == 0) ? phase_a<V, true>(a, bc, pold, pnew, 0.0f, t0, stride)
                                  : phase_a<V, false>(a, bc, pold, pnew, s_pal, t0, stride);
-      s = block_sum_all(pw);
-      if (threadIdx.x == 0) q0[bid] = s;
-      if (!grid_sync(a.st, G)) return;
-      const double dpi = reduce_partials(q0, G);
+      s1[0] = pw;
+      if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
+      const double dpi = s1[0];
       if (!(dpi > 0.0)) break;  // inner breakdown: keep d, the FP64 sweep decides
       const float al = static_cast<float>(beta / dpi);
       betaold = beta;
@@ -574,14 +561,11 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
         __syncthreads();
       }
       }
-      s = block_sum_all(zz);
-      if (threadIdx.x == 0) q1[bid] = s;
-      s = block_sum_all(zr);
-      if (threadIdx.x == 0) q2[bid] = s;
-      if (!grid_sync(a.st, G)) return;
-      const double zn = sqrt(reduce_partials(q1, G));
+      double s2[2] = {zz, zr};
+      if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+      const double zn = sqrt(s2[0]);
       if (zn <= itol) break;
-      beta = reduce_partials(q2, G);
+      beta = s2[1];
     }
   }
   // The solution of the last outer pass lives in x1 after even passes.
@@ -597,17 +581,8 @@ __device__ __forceinline__ void cg_mixed_body(const MixedArgs& a, const int bid,
   }
 }
 
-// Blocks per SM of the mixed solves: as many as fit without register spills
-// (three; two for 8 cells per lane and for the batched forms, whose member
-// records add registers).  At four the 64-register cap spilled 126 bytes a
-// thread and the 512x512x128 solve ran 5 % slower (12.5 against 11.8 ms).
 template <int V, int E>
-constexpr int mixed_min_blocks(bool batch) {
-  return (E == 8 || (batch && (V == 4 || E == 8))) ? 2 : 3;
-}
-
-template <int V, int E>
-__global__ void __launch_bounds__(kCgBlock, mixed_min_blocks<V, E>(false)) k_cg_mixed(MixedArgs a) {
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg_mixed(MixedArgs a) {
   cg_mixed_body<V, E>(a, blockIdx.x, gridDim.x);
 }
 
@@ -628,7 +603,7 @@ __device__ __forceinline__ void cg_mixed_any(const MixedArgs& a, int e, int sb, 
   }
 }
 
-__global__ void __launch_bounds__(kCgBlock, 2)
+__global__ void __launch_bounds__(kCgBlock, 1)
     k_cg_mixed_batch(const MixedArgs* __restrict__ tab, const int* __restrict__ first, int n,
                      int* queue, const int* __restrict__ order, const int* __restrict__ ofirst) {
   __shared__ MixedArgs sa;
@@ -761,12 +736,13 @@ cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, doub
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kCgBlock, ksm);
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  // 3 x g reduction partials fit the 4 x sm_count x 4 doubles allocated at create.
+  // the reduction slots allocated at create serve up to 4 sm_count blocks
   if (per_sm > 4) per_sm = 4;
   long long g = static_cast<long long>(per_sm) * D.sm_count;
   if (!wcol && g > ntiles) g = ntiles;
   if (g < 1) g = 1;
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * g, D.stream);
   MixedArgs a = make_mixed_args(D, atol, maxit, outer_rtol, max_outer);
   void* args[] = {&a};
   ++D.launches;

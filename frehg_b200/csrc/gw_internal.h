@@ -22,8 +22,7 @@ struct CgState {
   int reason;       // KSPConvergedReason (>0 converged, <0 diverged)
   int outer;        // defect-correction sweeps (mixed precision)
   int err;          // barrier timeout flag (0 = none)
-  unsigned bar_count;
-  unsigned bar_gen;
+  unsigned arrived; // blocks counted in at the solve's barriers (coop::grid_sum)
 };
 
 // Step results assembled on the device by k_step_info.
@@ -61,6 +60,9 @@ enum PartialSlot {
 // Launch geometry of the reducing cell kernels (fixed per domain so every
 // reduction has the same shape, and therefore the same rounding, each step).
 constexpr int kBlock = 256;
+
+// Reduction slots (doubles) a solve block needs (coop::grid_sum).
+constexpr size_t kSolveSlots = 8;
 
 struct Device {
   Dims d{};
@@ -121,7 +123,7 @@ struct Device {
   double *dinv64 = nullptr, *l64 = nullptr, *d64 = nullptr;
   // reductions
   double* partial = nullptr;   // kPSlots x nblk
-  double* cgpart = nullptr;    // 4 x cg grid
+  double* cgpart = nullptr;    // coop::kRedSlots x cg grid: the solves' reduction slots
   int nblk = 0;                // grid of the reducing cell kernels
   int cg_grid = 0;             // co-resident grid of the CG kernel
   int cg_grid32 = 0;
@@ -272,6 +274,7 @@ struct SolveGroup {
   void* tab = nullptr;           // device table of per-member kernel arguments
   int* first = nullptr;          // device block offsets, n + 1
   CgState** states = nullptr;    // device array of the members' CG states
+  double** parts = nullptr;      // device array of the members' reduction slots
   int* queue = nullptr;          // device counter of the slots handed out
   int* order = nullptr;          // device queue order of the members, n
   int* ofirst = nullptr;         // device slot offsets in queue order, n + 1
