@@ -8,23 +8,36 @@
 // 1e5 ||D^-1 b||, non-finite norms, indefinite matrix / preconditioner and
 // max_iterations.
 //
-// One persistent cooperative launch runs the whole solve.  Per iteration:
-//   phase A: p_new = z + b p_old (for the seven stencil points), w = A p_new,
-//            partial p'w;
+// The recurrences run on the system scaled to a unit diagonal: with
+// S = D^(-1/2), Jacobi-preconditioned CG on A x = b is plain CG on
+// (S A S) y = S b, x = S y, step for step (r' = S r, p' = S^-1 p, and z'r is
+// r'.r'), so the diagonal and z drop out of the iteration.
+//
+// One persistent cooperative launch runs the whole solve.  It scales the legs
+// in place, then per iteration:
+//   phase A: p_new = r + b p_old (for the seven stencil points), w = A p_new,
+//            partial p'w; every second iteration y += the last two a p;
 //   grid barrier that sums the partials (grid_sum);
-//   phase B: x += a p, r -= a w, z = r / diag, partials z'z and z'r;
+//   phase B: r -= a w, partials r'r and ||S r||^2 = ||D^-1 r||^2 (unscaled);
 //   the same barrier; convergence test.
 // Every thread takes two consecutive cells (cg64v_body), with 16-byte pair
 // loads where nz is even and separate loads where it is odd.
-// Per cell and iteration this moves 16 FP64 words (128 B) through HBM:
-// phase A reads z, p_old, diag, gxp, gyp, gzp and writes p_new, w; phase B
-// reads x, p_new, r, w, diag and writes x, r, z.  Neighbour reads are served
-// by L1/L2 because the grid-stride sweep keeps all resident blocks inside a
-// few j-rows of each other.
+// Per cell and iteration this moves 12.5 FP64 words (100 B): phase A reads r,
+// p_old, gxp, gyp, gzp and writes p_new, w, and half the time reads y and the
+// p before p_old (in p_new's buffer) and writes y; phase B reads r, w, s and
+// writes r.  Unscaled, with x updated every iteration and z stored, it was 16.
+// Neighbour reads are served by L1/L2 because the grid-stride sweep keeps all
+// resident blocks inside a few j-rows of each other.
+//
+// A thread's cells stay its own for the whole solve, so the words only it
+// reads can stay in shared memory (cg64_words: as many of w, y, s and the legs
+// as the domain's size leaves room for).  512x512x128 (no room) 692 -> 571 us an
+// iteration, 131x113x127 (w) 48.2 -> 36.7, 64x64x128 (four) 12.7 -> 11.0.
 //
 // The grid barrier's wait is bounded: one that exceeds kSpinLimit polls sets
 // CgState::err, and every block leaves at its next barrier, so a launch that
 // lost co-residency ends with an error status instead of hanging.
+#include <algorithm>
 #include <cfloat>
 #include <cstdio>
 #include <cstring>
@@ -40,8 +53,9 @@ using namespace coop;
 
 struct Cg64Args {
   Dims d;
-  const double *diag, *gxp, *gyp, *gzp, *b;
-  double *x, *r, *z, *p0, *p1, *w;
+  const double *diag, *b;
+  double *gxp, *gyp, *gzp;       // scaled in place
+  double *x, *r, *z, *p0, *p1, *w;  // x holds y and z holds s until the end
   double* part;  // kRedSlots x G, zero before the launch
   CgState* st;
   double rtol, atol;
@@ -49,17 +63,17 @@ struct Cg64Args {
   int variant;  // batched solves: 1 = 16-byte pair accesses (nz even), 0 = separate loads
 };
 
+// Up to this many pairs one block solves alone, without the grid barrier.
+constexpr long long kCgAlone = 2 * kCgBlock;
+
 __device__ inline int sgn(double v) { return (v > 0.0) - (v < 0.0); }
 
-// The same solve with two consecutive cells per thread.  With ALIGNED (nz
-// even, so every pair and every i/j-neighbour pair is 16-byte aligned) the
-// pairs move as 16-byte loads and stores: half the load instructions per cell
-// and twice the bytes in flight per request.  Otherwise (nz odd) the pair's
-// two cells load separately, still two cells' loads in flight per thread, and
-// an odd cell count leaves a last cell that one thread takes alone.  The
-// arithmetic per cell is the one-cell-per-thread form's (cg64_cell_*, which
-// also take that last cell); against it, the separate-load pairs took a
-// 256x256x127 solve from 95.4 to 57 ms.
+// Two consecutive cells per thread.  With ALIGNED (nz even, so every pair and
+// every i/j-neighbour pair is 16-byte aligned) the pairs move as 16-byte loads
+// and stores: half the load instructions per cell and twice the bytes in
+// flight per request.  Otherwise (nz odd) the pair's two cells load
+// separately, still two cells' loads in flight per thread, and an odd cell
+// count leaves a last cell that one thread takes alone (cg64_cell_*).
 __device__ inline double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 __device__ inline void st2(double* p, double a, double b) {
   *reinterpret_cast<double2*>(p) = make_double2(a, b);
@@ -82,56 +96,129 @@ __device__ inline void stp(double* p, double a, double b) {
   }
 }
 
-// The three per-cell steps of one cell alone (the order of terms of the pair
-// code), for the last cell of an odd count.
-__device__ inline void cg64_cell_init(const Cg64Args& a, long long c, double& zz, double& zr) {
-  const double rc = a.b[c];
+// The steps of one cell alone (the order of terms of the pair code), for the
+// last cell of an odd count.
+__device__ inline void cg64_cell_init(const Cg64Args& a, long long c, double& rr, double& zz) {
+  const double s = 1.0 / sqrt(a.diag[c]);
+  const double r = s * a.b[c];
   a.x[c] = 0.0;
-  a.r[c] = rc;
   a.p0[c] = 0.0;
-  a.p1[c] = 0.0;
-  const double z = rc * (1.0 / a.diag[c]);
-  a.z[c] = z;
-  zz += z * z;
-  zr += z * rc;
+  a.r[c] = r;
+  a.z[c] = s;
+  a.gxp[c] *= s / sqrt(a.diag[c + a.d.sx]);
+  a.gyp[c] *= s / sqrt(a.diag[c + a.d.sy]);
+  a.gzp[c] *= s / sqrt(a.diag[c + 1]);
+  rr += r * r;
+  zz += (s * r) * (s * r);
 }
-__device__ inline void cg64_cell_stencil(const Cg64Args& a, long long c, double bc,
-                                         const double* __restrict__ pold,
-                                         double* __restrict__ pnew, double& pw) {
+__device__ inline void cg64_cell_stencil(const Cg64Args& a, long long c, bool first, bool yup,
+                                         double bc, double al1, double al2, const double* pold,
+                                         double* pnew, double& pw) {
   const long long sx = a.d.sx, sy = a.d.sy;
-  const double pc = a.z[c] + bc * pold[c];
-  const double pym = a.z[c - sy] + bc * pold[c - sy];
-  const double pxm = a.z[c - sx] + bc * pold[c - sx];
-  const double pzm = a.z[c - 1] + bc * pold[c - 1];
-  const double pzp = a.z[c + 1] + bc * pold[c + 1];
-  const double pxp = a.z[c + sx] + bc * pold[c + sx];
-  const double pyp = a.z[c + sy] + bc * pold[c + sy];
-  double wv = a.gyp[c - sy] * pym;
-  wv += a.gxp[c - sx] * pxm;
-  wv += a.gzp[c - 1] * pzm;
-  wv += a.diag[c] * pc;
-  wv += a.gzp[c] * pzp;
-  wv += a.gxp[c] * pxp;
-  wv += a.gyp[c] * pyp;
+  const auto pv = [&](long long m) { return first ? a.r[m] : a.r[m] + bc * pold[m]; };
+  const double pc = pv(c);
+  double wv = a.gyp[c - sy] * pv(c - sy);
+  wv += a.gxp[c - sx] * pv(c - sx);
+  wv += a.gzp[c - 1] * pv(c - 1);
+  wv += pc;
+  wv += a.gzp[c] * pv(c + 1);
+  wv += a.gxp[c] * pv(c + sx);
+  wv += a.gyp[c] * pv(c + sy);
+  if (yup) a.x[c] += al1 * pold[c] + al2 * pnew[c];
   pnew[c] = pc;
   a.w[c] = wv;
   pw += pc * wv;
 }
-__device__ inline void cg64_cell_update(const Cg64Args& a, long long c, double al,
-                                        const double* __restrict__ pnew, double& zz,
-                                        double& zr) {
-  const double pc = pnew[c];
-  a.x[c] += al * pc;
-  const double rc = a.r[c] - al * a.w[c];
-  a.r[c] = rc;
-  const double z = rc * (1.0 / a.diag[c]);
-  a.z[c] = z;
+__device__ inline void cg64_cell_update(const Cg64Args& a, long long c, double al, double& rr,
+                                        double& zz) {
+  const double r = a.r[c] - al * a.w[c];
+  const double z = a.z[c] * r;
+  a.r[c] = r;
+  rr += r * r;
   zz += z * z;
-  zr += z * rc;
 }
 
-template <bool ALIGNED>
-__device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, const int G) {
+// The words of a thread's own cells held in shared memory, by what keeping
+// each saves in traffic: W of them, in this order.
+enum OwnWord { kOwnW = 0, kOwnY = 1, kOwnS = 2, kOwnGym = 3, kOwnGxm = 4, kOwnGx = 5, kOwnGy = 6 };
+
+// Phase A over a block's cells.  FIRST: p_new = r, p_old is not read, and the
+// legs held on chip are filled.  YUP: y takes the two pending updates.
+template <bool ALIGNED, int W, bool FIRST, bool YUP>
+__device__ __forceinline__ double cg64_phase_a(const Cg64Args& a, double2* __restrict__ own,
+                                               const int words, double bc, double al1, double al2,
+                                               const double* pold, double* pnew, long long t0,
+                                               long long stride) {
+  const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy;
+  // Local copies: a batched solve's record lies in shared memory, and a store
+  // through any of its pointers would have every pointer read again.
+  const double *const r = a.r, *const gxp = a.gxp, *const gyp = a.gyp, *const gzp = a.gzp;
+  double *const x = a.x, *const w = a.w;
+  double pw = 0.0;
+  int o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
+    const long long c = 2 * q;
+    const auto chip = [&](int word) -> double2& { return own[word * words + o]; };
+    const auto leg = [&](int word, const double* g) {
+      if (W > word && !FIRST) return chip(word);
+      const double2 v = ldp<ALIGNED>(g);
+      if (W > word) chip(word) = v;
+      return v;
+    };
+    const double2 zero = make_double2(0.0, 0.0);
+    const double2 rc = ldp<ALIGNED>(r + c);
+    const double2 pc = FIRST ? zero : ldp<ALIGNED>(pold + c);
+    const double2 rxm = ldp<ALIGNED>(r + c - sx), rxp = ldp<ALIGNED>(r + c + sx);
+    const double2 rym = ldp<ALIGNED>(r + c - sy), ryp = ldp<ALIGNED>(r + c + sy);
+    const double2 pxm = FIRST ? zero : ldp<ALIGNED>(pold + c - sx);
+    const double2 pxp = FIRST ? zero : ldp<ALIGNED>(pold + c + sx);
+    const double2 pym = FIRST ? zero : ldp<ALIGNED>(pold + c - sy);
+    const double2 pyp = FIRST ? zero : ldp<ALIGNED>(pold + c + sy);
+    const double rkm = r[c - 1], rkp = r[c + 2];
+    const double pkm = FIRST ? 0.0 : pold[c - 1], pkp = FIRST ? 0.0 : pold[c + 2];
+    const double2 gx = leg(kOwnGx, gxp + c), gxm = leg(kOwnGxm, gxp + c - sx);
+    const double2 gy = leg(kOwnGy, gyp + c), gym = leg(kOwnGym, gyp + c - sy);
+    const double2 gz = ldp<ALIGNED>(gzp + c);
+    const double gzm = gzp[c - 1];
+    double2 y = zero, pp = zero;
+    if (YUP) {
+      y = W > kOwnY ? chip(kOwnY) : ldp<ALIGNED>(x + c);
+      pp = ldp<ALIGNED>(pnew + c);
+    }
+    const double P0 = rc.x + bc * pc.x, P1 = rc.y + bc * pc.y;
+    double w0 = gym.x * (rym.x + bc * pym.x);
+    w0 += gxm.x * (rxm.x + bc * pxm.x);
+    w0 += gzm * (rkm + bc * pkm);
+    w0 += P0;
+    w0 += gz.x * P1;
+    w0 += gx.x * (rxp.x + bc * pxp.x);
+    w0 += gy.x * (ryp.x + bc * pyp.x);
+    double w1 = gym.y * (rym.y + bc * pym.y);
+    w1 += gxm.y * (rxm.y + bc * pxm.y);
+    w1 += gz.x * P0;
+    w1 += P1;
+    w1 += gz.y * (rkp + bc * pkp);
+    w1 += gx.y * (rxp.y + bc * pxp.y);
+    w1 += gy.y * (ryp.y + bc * pyp.y);
+    stp<ALIGNED>(pnew + c, P0, P1);
+    if (W > kOwnW) chip(kOwnW) = make_double2(w0, w1);
+    else stp<ALIGNED>(w + c, w0, w1);
+    if (YUP) {
+      y.x += al1 * pc.x + al2 * pp.x;
+      y.y += al1 * pc.y + al2 * pp.y;
+      if (W > kOwnY) chip(kOwnY) = y;
+      else stp<ALIGNED>(x + c, y.x, y.y);
+    }
+    pw += P0 * w0;
+    pw += P1 * w1;
+  }
+  return pw;
+}
+
+// W words of every own cell in shared memory (own, `words` pairs apart).
+template <bool ALIGNED, int W>
+__device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, const int G,
+                                           double2* __restrict__ own, const int words) {
   const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy;
   // The last cell of an odd count, taken by the grid's last thread.
   const bool tail = !ALIGNED && (a.d.ncell & 1) && bid == G - 1 &&
@@ -140,25 +227,40 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   const long long stride = static_cast<long long>(G) * blockDim.x;
   const long long t0 = bid * static_cast<long long>(blockDim.x) + threadIdx.x;
   unsigned epoch = 0;
+  double *const gxp = a.gxp, *const gyp = a.gyp, *const gzp = a.gzp, *const ra = a.r,
+               *const xa = a.x, *const wa = a.w, *const sa = a.z;
+  const double *const diag = a.diag, *const b = a.b;
 
-  double zz = 0.0, zr = 0.0;
-  for (long long q = t0; q < N2; q += stride) {
+  // Scale: s, r = S b, the legs in place (only their own cell's thread reads
+  // or writes them here); y = 0, p_(-1) = 0.
+  double rr = 0.0, zz = 0.0;
+  int o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
-    const double2 rc = ldp<ALIGNED>(a.b + c);
-    const double2 dg = ldp<ALIGNED>(a.diag + c);
-    stp<ALIGNED>(a.x + c, 0.0, 0.0);
-    stp<ALIGNED>(a.r + c, rc.x, rc.y);
+    const double2 bv = ldp<ALIGNED>(b + c), dg = ldp<ALIGNED>(diag + c);
+    const double2 dx = ldp<ALIGNED>(diag + c + sx), dy = ldp<ALIGNED>(diag + c + sy);
+    const double dz = diag[c + 2];
+    const double2 gx = ldp<ALIGNED>(gxp + c), gy = ldp<ALIGNED>(gyp + c);
+    const double2 gz = ldp<ALIGNED>(gzp + c);
+    const double s0 = 1.0 / sqrt(dg.x), s1 = 1.0 / sqrt(dg.y);
+    const double r0 = s0 * bv.x, r1 = s1 * bv.y;
+    stp<ALIGNED>(gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
+    stp<ALIGNED>(gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
+    stp<ALIGNED>(gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
+    stp<ALIGNED>(ra + c, r0, r1);
     stp<ALIGNED>(a.p0 + c, 0.0, 0.0);
-    stp<ALIGNED>(a.p1 + c, 0.0, 0.0);
-    const double z0 = rc.x * (1.0 / dg.x), z1 = rc.y * (1.0 / dg.y);
-    stp<ALIGNED>(a.z + c, z0, z1);
+    if (W > kOwnS) own[kOwnS * words + o] = make_double2(s0, s1);
+    else stp<ALIGNED>(sa + c, s0, s1);
+    if (W > kOwnY) own[kOwnY * words + o] = make_double2(0.0, 0.0);
+    else stp<ALIGNED>(xa + c, 0.0, 0.0);
+    const double z0 = s0 * r0, z1 = s1 * r1;
+    rr += r0 * r0;
+    rr += r1 * r1;
     zz += z0 * z0;
     zz += z1 * z1;
-    zr += z0 * rc.x;
-    zr += z1 * rc.y;
   }
-  if (tail) cg64_cell_init(a, ct, zz, zr);
-  double s2[2] = {zz, zr};
+  if (tail) cg64_cell_init(a, ct, rr, zz);
+  double s2[2] = {zz, rr};
   if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
   double dp = sqrt(s2[0]);
   double beta = s2[1];
@@ -172,7 +274,8 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   };
   test(dp);
   double betaold = 1.0, dpi = 0.0, dpiold = 0.0;
-  int i = 0;
+  double al = 0.0, al1 = 0.0;  // a of the last two iterations
+  int i = 0, done = -1;        // done: the last iteration whose a is known
   while (reason == 0) {
     its = i + 1;
     if (beta == 0.0) {
@@ -184,49 +287,16 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       break;
     }
     const double bc = (i == 0) ? 0.0 : beta / betaold;
-    const double* __restrict__ pold = (i & 1) ? a.p1 : a.p0;
-    double* __restrict__ pnew = (i & 1) ? a.p0 : a.p1;
-    double pw = 0.0;
-    for (long long q = t0; q < N2; q += stride) {
-      const long long c = 2 * q;
-      const double2 zc = ldp<ALIGNED>(a.z + c), pc = ldp<ALIGNED>(pold + c);
-      const double2 zxm = ldp<ALIGNED>(a.z + c - sx), pxm = ldp<ALIGNED>(pold + c - sx);
-      const double2 zxp = ldp<ALIGNED>(a.z + c + sx), pxp = ldp<ALIGNED>(pold + c + sx);
-      const double2 zym = ldp<ALIGNED>(a.z + c - sy), pym = ldp<ALIGNED>(pold + c - sy);
-      const double2 zyp = ldp<ALIGNED>(a.z + c + sy), pyp = ldp<ALIGNED>(pold + c + sy);
-      const double zkm = a.z[c - 1], pkm = pold[c - 1];
-      const double zkp = a.z[c + 2], pkp = pold[c + 2];
-      const double2 dg = ldp<ALIGNED>(a.diag + c);
-      const double2 gx = ldp<ALIGNED>(a.gxp + c), gxm = ldp<ALIGNED>(a.gxp + c - sx);
-      const double2 gy = ldp<ALIGNED>(a.gyp + c), gym = ldp<ALIGNED>(a.gyp + c - sy);
-      const double2 gz = ldp<ALIGNED>(a.gzp + c);
-      const double gzm = a.gzp[c - 1];
-      const double P0 = zc.x + bc * pc.x, P1 = zc.y + bc * pc.y;
-      const double Pkm = zkm + bc * pkm, Pkp = zkp + bc * pkp;
-      const double Pxm0 = zxm.x + bc * pxm.x, Pxm1 = zxm.y + bc * pxm.y;
-      const double Pxp0 = zxp.x + bc * pxp.x, Pxp1 = zxp.y + bc * pxp.y;
-      const double Pym0 = zym.x + bc * pym.x, Pym1 = zym.y + bc * pym.y;
-      const double Pyp0 = zyp.x + bc * pyp.x, Pyp1 = zyp.y + bc * pyp.y;
-      double w0 = gym.x * Pym0;
-      w0 += gxm.x * Pxm0;
-      w0 += gzm * Pkm;
-      w0 += dg.x * P0;
-      w0 += gz.x * P1;
-      w0 += gx.x * Pxp0;
-      w0 += gy.x * Pyp0;
-      double w1 = gym.y * Pym1;
-      w1 += gxm.y * Pxm1;
-      w1 += gz.x * P0;
-      w1 += dg.y * P1;
-      w1 += gz.y * Pkp;
-      w1 += gx.y * Pxp1;
-      w1 += gy.y * Pyp1;
-      stp<ALIGNED>(pnew + c, P0, P1);
-      stp<ALIGNED>(a.w + c, w0, w1);
-      pw += P0 * w0;
-      pw += P1 * w1;
-    }
-    if (tail) cg64_cell_stencil(a, ct, bc, pold, pnew, pw);
+    const double* pold = (i & 1) ? a.p1 : a.p0;
+    double* pnew = (i & 1) ? a.p0 : a.p1;
+    double pw;
+    if (i == 0)
+      pw = cg64_phase_a<ALIGNED, W, true, false>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
+    else if (i & 1)
+      pw = cg64_phase_a<ALIGNED, W, false, true>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
+    else
+      pw = cg64_phase_a<ALIGNED, W, false, false>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
+    if (tail) cg64_cell_stencil(a, ct, i == 0, (i & 1) != 0, bc, al, al1, pold, pnew, pw);
     double s1[1] = {pw};
     if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
     dpiold = dpi;
@@ -236,26 +306,28 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       reason = -10;
       break;
     }
-    const double al = beta / dpi;
+    al1 = al;
+    al = beta / dpi;
+    done = i;
+    rr = 0.0;
     zz = 0.0;
-    zr = 0.0;
-    for (long long q = t0; q < N2; q += stride) {
+    o = threadIdx.x;
+    for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
       const long long c = 2 * q;
-      const double2 pc = ldp<ALIGNED>(pnew + c), xc = ldp<ALIGNED>(a.x + c), rc0 = ldp<ALIGNED>(a.r + c);
-      const double2 wc = ldp<ALIGNED>(a.w + c), dg = ldp<ALIGNED>(a.diag + c);
-      stp<ALIGNED>(a.x + c, xc.x + al * pc.x, xc.y + al * pc.y);
-      const double r0 = rc0.x - al * wc.x, r1 = rc0.y - al * wc.y;
-      stp<ALIGNED>(a.r + c, r0, r1);
-      const double z0 = r0 * (1.0 / dg.x), z1 = r1 * (1.0 / dg.y);
-      stp<ALIGNED>(a.z + c, z0, z1);
+      const double2 r = ldp<ALIGNED>(ra + c);
+      const double2 w = W > kOwnW ? own[kOwnW * words + o] : ldp<ALIGNED>(wa + c);
+      const double2 s = W > kOwnS ? own[kOwnS * words + o] : ldp<ALIGNED>(sa + c);
+      const double r0 = r.x - al * w.x, r1 = r.y - al * w.y;
+      stp<ALIGNED>(ra + c, r0, r1);
+      const double z0 = s.x * r0, z1 = s.y * r1;
+      rr += r0 * r0;
+      rr += r1 * r1;
       zz += z0 * z0;
       zz += z1 * z1;
-      zr += z0 * r0;
-      zr += z1 * r1;
     }
-    if (tail) cg64_cell_update(a, ct, al, pnew, zz, zr);
+    if (tail) cg64_cell_update(a, ct, al, rr, zz);
     s2[0] = zz;
-    s2[1] = zr;
+    s2[1] = rr;
     if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
     dp = sqrt(s2[0]);
     test(dp);
@@ -267,6 +339,25 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       break;
     }
   }
+  // x = S y with the pending updates: iteration `done`'s and, where its own
+  // phase A did not apply the one before (even), that one's.
+  const double e1 = done < 0 ? 0.0 : al, e2 = (done > 0 && !(done & 1)) ? al1 : 0.0;
+  const double* pl = (done & 1) ? a.p0 : a.p1;
+  const double* pv = (done & 1) ? a.p1 : a.p0;
+  const auto fin = [&](double s, double y, long long c) {
+    if (done >= 0) y += e1 * pl[c];
+    if (e2 != 0.0) y += e2 * pv[c];
+    xa[c] = s * y;
+  };
+  o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
+    const long long c = 2 * q;
+    const double2 s = W > kOwnS ? own[kOwnS * words + o] : ldp<ALIGNED>(sa + c);
+    const double2 y = W > kOwnY ? own[kOwnY * words + o] : ldp<ALIGNED>(xa + c);
+    fin(s.x, y.x, c);
+    fin(s.y, y.y, c + 1);
+  }
+  if (tail) fin(sa[ct], xa[ct], ct);
   if (bid == 0 && threadIdx.x == 0) {
     a.st->dp = dp;
     a.st->rnorm0 = rnorm0;
@@ -278,12 +369,10 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
 
 // 128 registers a thread: at an 80-register cap (768 threads per SM) the
 // kernel spilled and the 512x512x128 FP64 solve took 251 ms against 236.
-__global__ void __launch_bounds__(kCgBlock, 1) k_cg64v(Cg64Args a) {
-  cg64v_body<true>(a, blockIdx.x, gridDim.x);
-}
-
-__global__ void __launch_bounds__(kCgBlock, 1) k_cg64u(Cg64Args a) {
-  cg64v_body<false>(a, blockIdx.x, gridDim.x);
+template <bool ALIGNED, int W>
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg64(Cg64Args a, int words) {
+  extern __shared__ double2 own[];
+  cg64v_body<ALIGNED, W>(a, blockIdx.x, gridDim.x, own, words);
 }
 
 // One cooperative launch over several domains: instance i owns
@@ -313,9 +402,9 @@ __global__ void __launch_bounds__(kCgBlock, 1)
     __syncthreads();
     if (slot >= first[n]) break;
     if (sa.variant) {
-      cg64v_body<true>(sa, sb, sg);
+      cg64v_body<true, 0>(sa, sb, sg, nullptr, 0);
     } else {
-      cg64v_body<false>(sa, sb, sg);
+      cg64v_body<false, 0>(sa, sb, sg, nullptr, 0);
     }
     __syncthreads();  // every thread is done with sa before the next slot's
   }
@@ -323,17 +412,12 @@ __global__ void __launch_bounds__(kCgBlock, 1)
 
 }  // namespace
 
+// One block per SM; as few as hold a pair of cells a thread, and one alone
+// (no grid barrier) up to kCgAlone pairs.
 int cg64_grid(int sm_count, long long ncell) {
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg64u, kCgBlock, 0);
-  int per_sm_v = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_v, k_cg64v, kCgBlock, 0);
-  if (per_sm_v < per_sm) per_sm = per_sm_v;
-  if (per_sm < 1) per_sm = 1;
-  const long long want = (ncell + kCgBlock - 1) / kCgBlock;
-  long long g = static_cast<long long>(per_sm) * sm_count;
-  if (want < g) g = want;
-  return static_cast<int>(g < 1 ? 1 : g);
+  const long long pairs = ncell / 2;
+  if (pairs <= kCgAlone) return 1;
+  return static_cast<int>(std::min<long long>((pairs + kCgBlock - 1) / kCgBlock, sm_count));
 }
 
 namespace {
@@ -362,15 +446,43 @@ Cg64Args make_cg64_args(const Device& D, double rtol, double atol, int maxit) {
 
 }  // namespace
 
+namespace {
+
+// Shared-memory words of the own cells at `pairs` pairs a thread: the largest
+// built variant within kOwnBytes.  Half the SM's 256 KB stays L1, which serves
+// the stencil's neighbours: with 208 KB taken the 131x113x127 iteration was
+// 54.8 us against 37.0 with 104 KB and 40.5 with none (64x64x128: 224 KB 11.5,
+// 128 KB 10.9, none 11.4; 101x55x25, 56 KB: 5 % of a coupled pass).
+constexpr size_t kOwnBytes = 128 * 1024;
+int cg64_words(long long pairs) {
+  const long long fit = kOwnBytes / (pairs * kCgBlock * sizeof(double2));
+  return fit >= 7 ? 7 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 0;
+}
+
+using Cg64Kernel = void (*)(Cg64Args, int);
+template <bool ALIGNED>
+Cg64Kernel cg64_kernel(int w) {
+  return w == 7 ? k_cg64<ALIGNED, 7> : w == 4 ? k_cg64<ALIGNED, 4> : w == 2 ? k_cg64<ALIGNED, 2>
+       : w == 1 ? k_cg64<ALIGNED, 1> : k_cg64<ALIGNED, 0>;
+}
+
+}  // namespace
+
 cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit) {
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
-  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * D.cg_grid, D.stream);
   Cg64Args a = make_cg64_args(D, rtol, atol, maxit);
-  void* args[] = {&a};
+  const long long threads = static_cast<long long>(D.cg_grid) * kCgBlock;
+  const long long pairs = std::max<long long>(1, (D.d.ncell / 2 + threads - 1) / threads);
+  const int w = cg64_words(pairs);
+  int words = static_cast<int>(pairs * kCgBlock);
+  const size_t smem = w * words * sizeof(double2);
+  const void* kern = reinterpret_cast<const void*>((D.d.nz % 2 == 0) ? cg64_kernel<true>(w)
+                                                                     : cg64_kernel<false>(w));
+  const cudaError_t e = raise_smem_limit(kern, smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&a, &words};
   ++D.launches;
-  const void* kern = (D.d.nz % 2 == 0) ? reinterpret_cast<const void*>(k_cg64v)
-                                       : reinterpret_cast<const void*>(k_cg64u);
-  return cudaLaunchCooperativeKernel(kern, dim3(D.cg_grid), dim3(kCgBlock), args, 0, D.stream);
+  return cudaLaunchCooperativeKernel(kern, dim3(D.cg_grid), dim3(kCgBlock), args, smem, D.stream);
 }
 
 size_t cg64_args_bytes() { return sizeof(Cg64Args); }

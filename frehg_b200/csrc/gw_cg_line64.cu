@@ -311,7 +311,6 @@ cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rto
   if (per_sm > 4) per_sm = 4;
   const long long g = static_cast<long long>(per_sm) * D.sm_count;
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
-  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * g, D.stream);
   Line64Args a;
   a.d = D.d;
   a.diag = D.diag;

@@ -742,7 +742,6 @@ cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, doub
   if (!wcol && g > ntiles) g = ntiles;
   if (g < 1) g = 1;
   cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
-  cudaMemsetAsync(D.cgpart, 0, kRedSlots * sizeof(double) * g, D.stream);
   MixedArgs a = make_mixed_args(D, atol, maxit, outer_rtol, max_outer);
   void* args[] = {&a};
   ++D.launches;

@@ -48,6 +48,20 @@ __device__ inline double warp_sum(double v) {
   return v;
 }
 
+// Sum of a block's warp sums, pairwise (a chain of 16 additions is 0.15 us).
+__device__ inline double tree_sum(const double* w) {
+  constexpr int kWarps = kCgBlock / 32;
+  double t[kWarps];
+#pragma unroll
+  for (int q = 0; q < kWarps; ++q) t[q] = w[q];
+#pragma unroll
+  for (int m = kWarps / 2; m > 0; m >>= 1) {
+#pragma unroll
+    for (int q = 0; q < m; ++q) t[q] += t[q + m];
+  }
+  return t[0];
+}
+
 // Grid barrier and sum in one exchange, for a cooperative (co-resident)
 // launch of kCgBlock threads a block: v[n] <- the sum of every thread's v[n]
 // over the G blocks, the same bits in every thread (fixed order: lanes, warps,
@@ -86,9 +100,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
     ++epoch;
     if (wid == 0) {
       if (lane < NV) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) s += sh[lane][w];
+        const double s = tree_sum(sh[lane]);
         st_relaxed_f64(gen + static_cast<long long>(lane) * G + bid, s);
       }
       __syncwarp();
@@ -126,18 +138,10 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
     }
     __syncthreads();
 #pragma unroll
-    for (int n = 0; n < NV; ++n) {
-      v[n] = 0.0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) v[n] += sw[n][w];
-    }
+    for (int n = 0; n < NV; ++n) v[n] = tree_sum(sw[n]);
   } else {
 #pragma unroll
-    for (int n = 0; n < NV; ++n) {
-      v[n] = 0.0;
-#pragma unroll
-      for (int w = 0; w < kWarps; ++w) v[n] += sh[n][w];
-    }
+    for (int n = 0; n < NV; ++n) v[n] = tree_sum(sh[n]);
     __syncthreads();
   }
   return true;

@@ -2628,9 +2628,12 @@ __global__ void k_gather_outs(const StepArgs* tab, StepOut* outs, int n) {
 // ---------------------------------------------------------------- launchers
 cudaError_t raise_smem_limit(const void* kernel, size_t bytes) {
   static std::mutex mu;
-  static std::map<const void*, size_t> limit;
+  static std::map<std::pair<int, const void*>, size_t> limit;  // the limit is per device
+  int dev = 0;
+  const cudaError_t ed = cudaGetDevice(&dev);
+  if (ed != cudaSuccess) return ed;
   std::lock_guard<std::mutex> lock(mu);
-  size_t& cur = limit[kernel];
+  size_t& cur = limit[{dev, kernel}];
   if (bytes <= cur) return cudaSuccess;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(bytes));
