@@ -515,7 +515,6 @@ cudaError_t enqueue_predictor(frehg_gw_handle* h, double dtg) {
   if (D.f.cpl) fgw::launch_cpl_mode(D, hn);
   const bool mixed = h->precision == FREHG_GW_PRECISION_MIXED;
   const bool line64 = h->precision == FREHG_GW_PRECISION_FP64_LINE;
-  if (!line64 && h->fused && fgw::launch_predict(D, hn, wcn, mixed)) return cudaGetLastError();
   fgw::launch_closure_pred(D, hn);
   // Both warm-started forms begin from h^n, or, when the previous step's
   // start state h^(n-1) is still in the other state buffer, from the linear
@@ -534,12 +533,10 @@ void enqueue_corrector(frehg_gw_handle* h) {
   const int nxt = 1 - D.cur;
   double* hn = D.h[D.cur];
   double* wcn = D.wc[D.cur];
-  if (!(h->fused && fgw::launch_correct(D, hn, wcn))) {
-    fgw::launch_closure_corr(D, hn);
-    fgw::launch_flux(D, wcn);
-    if (D.f.cpl) fgw::launch_cpl_book(D, wcn);
-    fgw::launch_update_wc(D, hn, wcn);
-  }
+  fgw::launch_closure_corr(D, hn);
+  fgw::launch_flux(D, wcn);
+  if (D.f.cpl) fgw::launch_cpl_book(D, wcn);
+  fgw::launch_update_wc(D, hn, wcn);
   if (h->profiling) cudaEventRecord(h->ev[3], D.stream);
   fgw::launch_classify(D, D.wc[nxt], D.h[nxt]);
   fgw::launch_walk(D, D.wc[nxt]);
@@ -825,9 +822,8 @@ int frehg_gw_set_profiling(frehg_gw_handle* h, int on) {
 int frehg_gw_set_fused(frehg_gw_handle* h, int on) {
   if (!h) return fail(FREHG_GW_EINVAL, "null handle");
   // The fused passes raised a misaligned-address error on the B200 whose
-  // cause is not found; they are not switched on until it is.
+  // cause was not found; they are not built.
   if (on) return fail(FREHG_GW_EUNSUPPORTED, "set_fused: the fused passes are disabled");
-  h->fused = false;
   return FREHG_GW_OK;
 }
 

@@ -26,7 +26,6 @@ struct frehg_gw_handle {
   bool have_state = false;
   int start_buf = 0;  // ping-pong index of the last step's theta^n
   bool profiling = false;
-  bool fused = false;  // fused phase kernels where they apply (frehg_gw_set_fused)
   // Starting iterate of the mixed / FP64 line solves (frehg_gw_set_warm_start):
   // extrapolated from the previous step's start state when it is at hand
   // (have_prev: the last call stepped this handle alone from that state).

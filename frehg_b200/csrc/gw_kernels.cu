@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(kBlock) k_closure_corr(Dims d, Fields f,
 // Everything the row of one active cell depends on, gathered before any
 // arithmetic: the six face conductivities, activity of the upper neighbours
 // and of the cells above and below, metrics, step-start state, BC data and
-// (density) the ratios.  Shared by k_assemble and the fused predictor.
+// (density) the ratios.  The rows of k_assemble.
 struct AsmIn {
   double kxp, kxm, kyp, kym, kzm, kzp;
   double dzc, dzu, dzl, wcnc, wcsc;
@@ -593,182 +593,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_faces(Dims d, Fields f, PassK pk,
   faces_body<CPL>(d, f, pk, kx, ky, kzf, blockIdx.x, gridDim.x);
 }
 
-// ---------------------------------------------------------------- fused predictor
-// The whole predictor of a groundwater-only domain (no coupled top, no
-// density coupling; nz <= 32 E) in one pass: the closures of h^n, the face
-// conductivities, the row assembly and, for the mixed form, the FP32 casts
-// and the column LDL^T factors -- the work of k_closure_pred, k_faces,
-// k_assemble and k_line_factor_warp without their intermediate arrays (per
-// cell K x3 and C, the three face arrays, the FP64 re-read by the factor).
-//
-// A block owns a strip of kPredCols interior columns along i plus one halo
-// column on each side, one warp per column, lane l holding the E consecutive
-// cells k = l E + e of it, and marches j over kPredRows rows.  At row j it
-// evaluates the closures of row j + 1 (K along x for the strip and its
-// halo, K along y for the strip into shared memory; K along z and C(h^n)
-// stay in registers for the next row), then every interior warp takes its
-// cell's six faces -- x from the shared row, y from the shared rows j - 1,
-// j, j + 1, z by shuffles along its own column -- and the row.  K along x
-// lives in three row slots and K along y in four, so a slot is rewritten
-// only after every warp has passed the barrier that follows its last
-// reader: one __syncthreads per row.  Halo columns cost 2 / kPredCols more
-// closures and each segment one more row; the closures are cheap against
-// the memory traffic.  The values are those of the separate passes: the
-// same closure, face-rule and row functions on the same inputs.
-constexpr int kPredWarps = 8;
-constexpr int kPredCols = kPredWarps - 2;
-constexpr int kPredRows = 16;
-
-// Shared memory of one block: K along x in three row slots for every warp,
-// K along y in four row slots and K along z and C(h^n) in two row slots for
-// the interior warps.
-__host__ __device__ inline size_t pred_smem_bytes(int E) {
-  return static_cast<size_t>(3 * kPredWarps + 4 * kPredCols + 4 * kPredCols) * 32 * E *
-         sizeof(double);
-}
-
-// Closures of row jj for warp w's column i (Predictor.cpp:127-232,
-// 445-452): K along x into its slot; with `ky` K along y, with `full` K
-// along z and C(h^n) into the interior column iw's slots.
-template <int E>
-__device__ __forceinline__ void pred_closures(const Dims& d, const Fields& f,
-                                              const double* __restrict__ hn, double* psm, int w,
-                                              int iw, int i, int jj, bool ky, bool full) {
-  constexpr int NZP = 32 * E;
-  double* kxs = psm + ((jj % 3) * kPredWarps + w) * NZP;
-  double* kys = psm + 3 * kPredWarps * NZP + ((jj & 3) * kPredCols + iw) * NZP;
-  double* kzs = psm + (3 * kPredWarps + 4 * kPredCols) * NZP + ((jj & 1) * kPredCols + iw) * NZP;
-  double* chs = psm + (3 * kPredWarps + 6 * kPredCols) * NZP + ((jj & 1) * kPredCols + iw) * NZP;
-  const int k0 = (threadIdx.x & 31) * E, nz = d.nz;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int k = k0 + e;
-    if (k < nz) {
-      const long long c = cidx(d, jj, i, k);
-      const double hc = hn[c];
-      const Soil so = soil_at(f, c);
-      const double ksx = f.ksx[c], ksy = f.ksy[c], ksz = f.ksz[c];
-      const VgParts v = vg_parts(so, hc);
-      const KrParts p = vg_kr_from(v, hc);
-      kxs[k] = vg_k_from(p, ksx);
-      if (ky) kys[k] = vg_k_from(p, ksy);
-      if (full) {
-        kzs[k] = vg_k_from(p, ksz);
-        chs[k] = vg_capacity_from(so, v, hc);
-      }
-    }
-  }
-}
-
-// Two blocks per SM up to 128 cells a column; deeper columns need 147 KB of
-// shared memory a block, one block per SM, with the registers that frees.
-// The kernel body takes the domain's Dims and Fields by value, as the other
-// cell kernels' bodies do.
-template <int E, bool MIXED>
-__device__ __forceinline__ void predict_body(
-    Dims d, Fields f, const double* __restrict__ hn, const double* __restrict__ wcn,
-    const double* __restrict__ dtgp, double* __restrict__ diag, double* __restrict__ gxps,
-    double* __restrict__ gyps, double* __restrict__ gzps, double* __restrict__ rhs,
-    double* __restrict__ xw, float* __restrict__ diag32, float* __restrict__ gxp32,
-    float* __restrict__ gyp32, float* __restrict__ gzp32, float* __restrict__ dinv32,
-    float* __restrict__ l32) {
-  extern __shared__ __align__(16) double psm[];
-  constexpr int NZP = 32 * E;
-  double* skx = psm;                                // [3][kPredWarps][NZP]
-  double* sky = skx + 3 * kPredWarps * NZP;         // [4][kPredCols][NZP]
-  double* skz = sky + 4 * kPredCols * NZP;          // [2][kPredCols][NZP]
-  double* sch = skz + 2 * kPredCols * NZP;          // [2][kPredCols][NZP]
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k0 = lane * E;
-  const int i = blockIdx.x * kPredCols + w;  // this warp's column (warp 0: the west halo)
-  const bool has_col = i <= d.nx + 1;
-  const bool inner = w >= 1 && w <= kPredCols && i <= d.nx;
-  const int iw = w - 1;  // index among the interior columns
-  const int jb = 1 + blockIdx.y * kPredRows;
-  const int je = min(d.ny, jb + kPredRows - 1);
-  const int nz = d.nz;
-  const double dtg = *dtgp;
-
-  if (has_col) {
-    if (inner) pred_closures<E>(d, f, hn, psm, w, iw, i, jb - 1, true, false);  // K along y
-    pred_closures<E>(d, f, hn, psm, w, iw, i, jb, inner, inner);
-  }
-  for (int j = jb; j <= je; ++j) {
-    if (has_col) pred_closures<E>(d, f, hn, psm, w, iw, i, j + 1, inner, inner);
-    __syncthreads();
-    if (inner) {
-      const double* kx0 = skx + ((j % 3) * kPredWarps) * NZP;
-      const double* kyS = sky + (((j - 1) & 3) * kPredCols + iw) * NZP;
-      const double* kyC = sky + ((j & 3) * kPredCols + iw) * NZP;
-      const double* kyN = sky + (((j + 1) & 3) * kPredCols + iw) * NZP;
-      const double* kzC = skz + ((j & 1) * kPredCols + iw) * NZP;
-      const double* chC = sch + ((j & 1) * kPredCols + iw) * NZP;
-      const long long col = col2(d, j, i), cb = cidx(d, j, i, 0);
-      const int topc = f.topc[col], botc = f.botc[col];
-      const int xcode_m = (i == 1) ? f.xmc[col2(d, j, 1)] : f.xpc[col2(d, j, d.nx)];
-      const int xcode_p = f.xpc[col2(d, j, d.nx)];
-      const int ycode_m = (j == 1) ? f.ymc[col2(d, 1, i)] : f.ypc[col2(d, d.ny, i)];
-      const int ycode_p = f.ypc[col2(d, d.ny, i)];
-      double av[E], ev[E], xv[E], yv[E];
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        const int k = k0 + e;
-        av[e] = 1.0;
-        ev[e] = xv[e] = yv[e] = 0.0;
-        if (k < nz) {
-          const long long c = cb + k;
-          const long long ce = c + d.sx, cw = c - d.sx, cn = c + d.sy, cs = c - d.sy;
-          const long long cu = (k >= 1) ? c - 1 : c, cl = (k + 1 < nz) ? c + 1 : c;
-          const double wcc = wcn[c], wsc = f.wcs[c];
-          const int8_t ac = f.act[c];
-          const Flank fc_x{kx0[w * NZP + k], f.ksx[c], wcc, wsc, ac};
-          const Flank fe_x{kx0[(w + 1) * NZP + k], f.ksx[ce], wcn[ce], f.wcs[ce], f.act[ce]};
-          const Flank fw_x{kx0[(w - 1) * NZP + k], f.ksx[cw], wcn[cw], f.wcs[cw], f.act[cw]};
-          const Flank fc_y{kyC[k], f.ksy[c], wcc, wsc, ac};
-          const Flank fn_y{kyN[k], f.ksy[cn], wcn[cn], f.wcs[cn], f.act[cn]};
-          const Flank fs_y{kyS[k], f.ksy[cs], wcn[cs], f.wcs[cs], f.act[cs]};
-          const ZFlank zu{(k >= 1) ? kzC[k - 1] : kzC[k], f.ksz[cu], f.dz[cu],
-                          (k >= 1) ? f.act[cu] : int8_t(0)};
-          const ZFlank zc{kzC[k], f.ksz[c], f.dz[c], ac};
-          const ZFlank zl{(k + 1 < nz) ? kzC[k + 1] : 0.0, f.ksz[cl], f.dz[cl],
-                          (k + 1 < nz) ? f.act[cl] : int8_t(0)};
-          AsmIn a;
-          a.kxp = face_lat(d, fc_x, fe_x, false, i == d.nx, xcode_p);
-          a.kxm = face_lat(d, fw_x, fc_x, i == 1, false, xcode_m);
-          a.kyp = face_lat(d, fc_y, fn_y, false, j == d.ny, ycode_p);
-          a.kym = face_lat(d, fs_y, fc_y, j == 1, false, ycode_m);
-          a.kzm = face_z<false>(d, zu, zc, k, topc, botc, 0.0);
-          if (k + 1 < nz) {
-            a.kzp = face_z<false>(d, zc, zl, k + 1, topc, botc, 0.0);
-          } else {
-            const ZFlank none{0.0, 0.0, 0.0, 0};
-            a.kzp = face_z<false>(d, zc, none, nz, topc, botc, 0.0);
-          }
-          assemble_gather<false, false>(d, f, hn, wcn, chC[k], c, j, i, k, a);
-          if (MIXED) xw[c] = ac ? a.hnc : 0.0;  // the mixed solve's starting iterate
-          double rv = 0.0;
-          if (ac) {
-            const AsmOut o = assemble_math<false, false>(d, a, dtg, j, i, k);
-            av[e] = o.diag;
-            xv[e] = o.gxp;
-            yv[e] = o.gyp;
-            ev[e] = o.gzp;
-            rv = o.rhs;
-          }
-          diag[c] = av[e];
-          gxps[c] = xv[e];
-          gyps[c] = yv[e];
-          gzps[c] = ev[e];
-          rhs[c] = rv;
-        }
-      }
-      if (MIXED) factor_column<E>(nz, cb, av, ev, xv, yv, diag32, gxp32, gyp32, gzp32, dinv32, l32);
-    }
-    // The next row's closures rewrite this warp's K along z and C slots
-    // that other lanes of the warp have just read.
-    __syncwarp();
-  }
-}
-
 // ---------------------------------------------------------------- fluxes
 // Corrector faces and Darcy fluxes (computeFaceConductivity from the predicted
 // head, Predictor.cpp:105-386, and computeFluxesImpl<PC, HARM>,
@@ -1096,264 +920,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_update_wc(
     uint8_t* __restrict__ satf, int* __restrict__ colflag, double* partial) {
   update_wc_body<BARO>(d, f, hp, hn, wcn, qx, qy, qzf, dtgp, wcu, satf, colflag, partial,
                        blockIdx.x, gridDim.x);
-}
-
-template <int E, bool MIXED>
-__global__ void __launch_bounds__(kPredWarps * 32, (E >= 8) ? 1 : 2) k_predict(
-    Dims d, Fields f, const double* __restrict__ hn, const double* __restrict__ wcn,
-    const double* __restrict__ dtgp, double* __restrict__ diag, double* __restrict__ gxps,
-    double* __restrict__ gyps, double* __restrict__ gzps, double* __restrict__ rhs,
-    double* __restrict__ xw, float* __restrict__ diag32, float* __restrict__ gxp32,
-    float* __restrict__ gyp32, float* __restrict__ gzp32, float* __restrict__ dinv32,
-    float* __restrict__ l32) {
-  predict_body<E, MIXED>(d, f, hn, wcn, dtgp, diag, gxps, gyps, gzps, rhs, xw, diag32, gxp32,
-                         gyp32, gzp32, dinv32, l32);
-}
-
-// ---------------------------------------------------------------- fused corrector
-// The corrector of a groundwater-only domain (no coupled top, no density
-// coupling; nz <= 32 E) in one pass: the head scatter with its ghosts and
-// the closures of the predicted head (k_closure_corr), the corrector's face
-// conductivities and Darcy fluxes (k_flux) and the theta update with the
-// saturation flags and the Ss audit partials (k_update_wc), without the
-// per-cell K arrays between them.  The same strip and row march as
-// k_predict: at row j the closures of row j + 1 fill the shared rows (the
-// predicted head and K along x for the strip and its halo, K along y for
-// the strip, K along z per warp), then every interior warp takes its cell's
-// six fluxes -- the x- and y- ones evaluated again from the same inputs as
-// the neighbour that owns and stores them -- and theta.  Ghost cells'
-// outputs (predicted head, theta, flags) are stored by the block that owns
-// the strip and rows they border, once.  The grid is the domain's reducing
-// grid (D.nblk blocks) walking the (strip, segment) items, so each block
-// leaves one Ss partial.
-constexpr int kCorrWarps = 8;
-constexpr int kCorrCols = kCorrWarps - 2;
-constexpr int kCorrRows = 16;
-
-__host__ __device__ inline size_t corr_smem_bytes(int E) {
-  // K along x [3][warps], head [4][warps], K along y [4][cols], K along z [2][cols]
-  return static_cast<size_t>(3 * kCorrWarps + 4 * kCorrWarps + 4 * kCorrCols + 2 * kCorrCols) *
-         32 * E * sizeof(double);
-}
-
-// The ghost cells an item of k_correct stores: its columns [.., ..] (own_i
-// for this warp's column) and rows [jlo, jhi].
-struct CorrOwn {
-  bool own_i;
-  int jlo, jhi;
-};
-
-// Closures of row jj for warp w's column i of k_correct: the predicted head
-// and K along x into their slots; with `ky` K along y, with `full` K along z
-// (interior column iw).  Ghost cells the item owns get their outputs (head,
-// theta^n as theta, the saturation flag, a cleared column flag).
-template <int E>
-__device__ __forceinline__ void corr_closures(const Dims& d, const Fields& f,
-                                              const double* __restrict__ x,
-                                              const double* __restrict__ hn,
-                                              const double* __restrict__ wcn, double* csm, int w,
-                                              int iw, int i, int jj, bool ky, bool full,
-                                              CorrOwn own, double* __restrict__ hp,
-                                              double* __restrict__ wcu, uint8_t* __restrict__ satf,
-                                              int* __restrict__ colflag) {
-  constexpr int NZP = 32 * E;
-  double* kxs = csm + ((jj % 3) * kCorrWarps + w) * NZP;
-  double* hps = csm + 3 * kCorrWarps * NZP + ((jj & 3) * kCorrWarps + w) * NZP;
-  double* kys = csm + 7 * kCorrWarps * NZP + ((jj & 3) * kCorrCols + iw) * NZP;
-  double* kzs = csm + (7 * kCorrWarps + 4 * kCorrCols) * NZP + ((jj & 1) * kCorrCols + iw) * NZP;
-  const bool ghost = jj == 0 || jj == d.ny + 1 || i == 0 || i == d.nx + 1;
-  const bool store = ghost && own.own_i && jj >= own.jlo && jj <= own.jhi;
-  const int k0 = (threadIdx.x & 31) * E, nz = d.nz;
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int k = k0 + e;
-    if (k < nz) {
-      const long long c = cidx(d, jj, i, k);
-      const Soil so = soil_at(f, c);
-      const double ksx = f.ksx[c], ksy = f.ksy[c], ksz = f.ksz[c];
-      const double hv = predicted_head(d, f, x, hn, c, jj, i);
-      const KrParts p = vg_kr_parts(so, hv);
-      hps[k] = hv;
-      kxs[k] = vg_k_from(p, ksx);
-      if (ky) kys[k] = vg_k_from(p, ksy);
-      if (full) kzs[k] = vg_k_from(p, ksz);
-      if (store) {
-        const double w0 = wcn[c];
-        hp[c] = hv;
-        wcu[c] = w0;
-        satf[c] = (w0 >= so.ts || hv > so.aev) ? 1 : 0;
-        if (k == 0) colflag[col2(d, jj, i)] = 0;
-      }
-    }
-  }
-}
-
-template <int E>
-__device__ __forceinline__ void correct_body(
-    Dims d, Fields f, const double* __restrict__ x, const double* __restrict__ hn,
-    const double* __restrict__ wcn, const double* __restrict__ dtgp, double* __restrict__ hp,
-    double* __restrict__ kx, double* __restrict__ ky, double* __restrict__ kzf,
-    double* __restrict__ qx, double* __restrict__ qy, double* __restrict__ qzf,
-    double* __restrict__ wcu, uint8_t* __restrict__ satf, int* __restrict__ colflag,
-    double* __restrict__ partial) {
-  extern __shared__ __align__(16) double csm[];
-  constexpr int NZP = 32 * E;
-  double* skx = csm;                               // [3][kCorrWarps][NZP]
-  double* shp = skx + 3 * kCorrWarps * NZP;        // [4][kCorrWarps][NZP]
-  double* sky = shp + 4 * kCorrWarps * NZP;        // [4][kCorrCols][NZP]
-  double* skz = sky + 4 * kCorrCols * NZP;         // [2][kCorrCols][NZP]
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k0 = lane * E;
-  const int iw = w - 1;
-  const int nz = d.nz;
-  const double dtg = *dtgp;
-  const int nstrips = (d.nx + kCorrCols - 1) / kCorrCols;
-  const int nitems = nstrips * ((d.ny + kCorrRows - 1) / kCorrRows);
-  double acc = 0.0;
-
-  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
-    const int strip = item % nstrips, seg = item / nstrips;
-    const int i0 = 1 + strip * kCorrCols;
-    const int i = i0 - 1 + w;
-    const bool has_col = i <= d.nx + 1;
-    const bool inner = w >= 1 && w <= kCorrCols && i <= d.nx;
-    const int jb = 1 + seg * kCorrRows;
-    const int je = min(d.ny, jb + kCorrRows - 1);
-    // the columns and rows whose ghost cells this item stores
-    const int ilo = (strip == 0) ? 0 : i0, ihi = min(d.nx, i0 + kCorrCols - 1);
-    const int ihi_g = (ihi == d.nx) ? d.nx + 1 : ihi;
-    const int jlo_g = (jb == 1) ? 0 : jb, jhi_g = (je == d.ny) ? d.ny + 1 : je;
-    const bool own_i = i >= ilo && i <= ihi_g;
-
-    __syncthreads();  // the previous item's last row is read before the slots are rewritten
-    const CorrOwn own{own_i, jlo_g, jhi_g};
-    if (has_col) {
-      corr_closures<E>(d, f, x, hn, wcn, csm, w, iw, i, jb - 1, inner, false, own, hp, wcu, satf,
-                       colflag);
-      corr_closures<E>(d, f, x, hn, wcn, csm, w, iw, i, jb, inner, inner, own, hp, wcu, satf,
-                       colflag);
-    }
-    for (int j = jb; j <= je; ++j) {
-      if (has_col)
-        corr_closures<E>(d, f, x, hn, wcn, csm, w, iw, i, j + 1, inner, inner, own, hp, wcu,
-                         satf, colflag);
-      __syncthreads();
-      if (inner) {
-        const double* kx0 = skx + ((j % 3) * kCorrWarps) * NZP;
-        const double* hp0 = shp + ((j & 3) * kCorrWarps) * NZP;
-        const double* hpS = shp + (((j - 1) & 3) * kCorrWarps + w) * NZP;
-        const double* hpN = shp + (((j + 1) & 3) * kCorrWarps + w) * NZP;
-        const double* kyS = sky + (((j - 1) & 3) * kCorrCols + iw) * NZP;
-        const double* kyC = sky + ((j & 3) * kCorrCols + iw) * NZP;
-        const double* kyN = sky + (((j + 1) & 3) * kCorrCols + iw) * NZP;
-        const double* kzC = skz + ((j & 1) * kCorrCols + iw) * NZP;
-        const long long col = col2(d, j, i), cb = cidx(d, j, i, 0), fb = fidx(d, j, i, 0);
-        const int topc = f.topc[col], botc = f.botc[col];
-        const double topv = f.topv[col], botv = f.botv[col];
-        const long long exm = col2(d, j, 1), exp_ = col2(d, j, d.nx);
-        const long long eym = col2(d, 1, i), eyp = col2(d, d.ny, i);
-        const int cxm = (i == 1) ? f.xmc[exm] : f.xpc[exp_], cxp = f.xpc[exp_];
-        const double vxm = (i == 1) ? f.xmv[exm] : f.xpv[exp_], vxp = f.xpv[exp_];
-        const int cym = (j == 1) ? f.ymc[eym] : f.ypc[eyp], cyp = f.ypc[eyp];
-        const double vym = (j == 1) ? f.ymv[eym] : f.ypv[eyp], vyp = f.ypv[eyp];
-        // one cell at a time: a cell's loads fill the registers
-#pragma unroll 1
-        for (int e = 0; e < E; ++e) {
-          const int k = k0 + e;
-          if (k >= nz) break;
-          const long long c = cb + k, fz = fb + k;
-          const long long ce = c + d.sx, cw = c - d.sx, cn = c + d.sy, cs = c - d.sy;
-          const long long cu = (k >= 1) ? c - 1 : c, cl = (k + 1 < nz) ? c + 1 : c;
-          const double hpc = hp0[w * NZP + k];
-          const double w0 = wcn[c], ts = f.wcs[c];
-          const int8_t ac = f.act[c];
-          const double botc_ = f.bot[c];
-          // lateral faces: c with its east / north neighbour (stored here),
-          // west / south neighbour with c (evaluated again)
-          const LatFlux vxe{kx0[w * NZP + k], kx0[(w + 1) * NZP + k], f.ksx[c], f.ksx[ce], hpc,
-                            hp0[(w + 1) * NZP + k], w0, wcn[ce], ts, f.wcs[ce], botc_, f.bot[ce],
-                            f.ax[c], f.cosx[c], f.sinx[c], ac, f.act[ce]};
-          const LatFlux vxw{kx0[(w - 1) * NZP + k], kx0[w * NZP + k], f.ksx[cw], f.ksx[c],
-                            hp0[(w - 1) * NZP + k], hpc, wcn[cw], w0, f.wcs[cw], ts, f.bot[cw],
-                            botc_, f.ax[cw], f.cosx[cw], f.sinx[cw], f.act[cw], ac};
-          const LatFlux vyn{kyC[k], kyN[k], f.ksy[c], f.ksy[cn], hpc, hpN[k], w0, wcn[cn], ts,
-                            f.wcs[cn], botc_, f.bot[cn], f.ay[c], f.cosy[c], f.siny[c], ac,
-                            f.act[cn]};
-          const LatFlux vys{kyS[k], kyC[k], f.ksy[cs], f.ksy[c], hpS[k], hpc, wcn[cs], w0,
-                            f.wcs[cs], ts, f.bot[cs], botc_, f.ay[cs], f.cosy[cs], f.siny[cs],
-                            f.act[cs], ac};
-          const double qxp = flux_lat(d, f, vxe, d.idx, false, i == d.nx, cxp, vxp, ce, 1.0, 1.0);
-          const double qxm = flux_lat(d, f, vxw, d.idx, i == 1, false, cxm, vxm, c, 1.0, 1.0);
-          const double qyp = flux_lat(d, f, vyn, d.idy, false, j == d.ny, cyp, vyp, cn, 1.0, 1.0);
-          const double qym = flux_lat(d, f, vys, d.idy, j == 1, false, cym, vym, c, 1.0, 1.0);
-          kx[c] = face_lat(d, Flank{vxe.kca, vxe.ksa, vxe.wa, vxe.wsa, vxe.acta},
-                           Flank{vxe.kcb, vxe.ksb, vxe.wb, vxe.wsb, vxe.actb}, false, i == d.nx,
-                           cxp);
-          qx[c] = qxp;
-          ky[c] = face_lat(d, Flank{vyn.kca, vyn.ksa, vyn.wa, vyn.wsa, vyn.acta},
-                           Flank{vyn.kcb, vyn.ksb, vyn.wb, vyn.wsb, vyn.actb}, false, j == d.ny,
-                           cyp);
-          qy[c] = qyp;
-          if (i == 1) {  // the west boundary face, in the ghost column's slot
-            kx[cw] = face_lat(d, Flank{vxw.kca, vxw.ksa, vxw.wa, vxw.wsa, vxw.acta},
-                              Flank{vxw.kcb, vxw.ksb, vxw.wb, vxw.wsb, vxw.actb}, true, false,
-                              cxm);
-            qx[cw] = qxm;
-          }
-          if (j == 1) {  // the south boundary face, in the ghost row's slot
-            ky[cs] = face_lat(d, Flank{vys.kca, vys.ksa, vys.wa, vys.wsa, vys.acta},
-                              Flank{vys.kcb, vys.ksb, vys.wb, vys.wsb, vys.actb}, true, false,
-                              cym);
-            qy[cs] = qym;
-          }
-          // z faces: above c (stored here) and below c (stored by the cell
-          // below, or here for the bottom face)
-          const double hpu = (k >= 1) ? hp0[w * NZP + k - 1] : hpc;
-          const ZFlank zu{(k >= 1) ? kzC[k - 1] : kzC[k], f.ksz[cu], f.dz[cu],
-                          (k >= 1) ? f.act[cu] : int8_t(0)};
-          const ZFlank zc{kzC[k], f.ksz[c], f.dz[c], ac};
-          kzf[fz] = face_z<false>(d, zu, zc, k, topc, botc, 0.0);
-          const double qzt = flux_zv(d, f, zu, zc, hpu, hpc, k, topc, topv, botc, botv, cu, 1.0, 1.0);
-          qzf[fz] = qzt;
-          double qzb;
-          if (k + 1 < nz) {
-            const ZFlank zl{kzC[k + 1], f.ksz[cl], f.dz[cl], f.act[cl]};
-            qzb = flux_zv(d, f, zc, zl, hpc, hp0[w * NZP + k + 1], k + 1, topc, topv, botc, botv,
-                          c, 1.0, 1.0);
-          } else {
-            const ZFlank none{0.0, 0.0, 0.0, 0};
-            kzf[fz + 1] = face_z<false>(d, zc, none, nz, topc, botc, 0.0);
-            qzb = flux_zv(d, f, zc, none, hpc, 0.0, nz, topc, topv, botc, botv, c, 1.0, 1.0);
-            qzf[fz + 1] = qzb;
-          }
-          double upd = w0;
-          if (ac)
-            upd = theta_update(d, dtg, w0, hpc, hn[c], zc.dz, ts, qxp, qxm, qyp, qym, qzt, qzb,
-                               acc);
-          hp[c] = hpc;
-          wcu[c] = upd;
-          satf[c] = (upd >= ts || hpc > f.aev[c]) ? 1 : 0;
-          if (k == 0) colflag[col] = 0;  // the walk's column flags start clear
-        }
-      }
-      // The next row's closures rewrite this warp's K along z slot, which
-      // other lanes of the warp have just read.
-      __syncwarp();
-    }
-  }
-  const double s = block_reduce(acc, SumOp(), 0.0);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
-}
-
-template <int E>
-__global__ void __launch_bounds__(kCorrWarps * 32, (E >= 8) ? 1 : 2) k_correct(
-    Dims d, Fields f, const double* __restrict__ x, const double* __restrict__ hn,
-    const double* __restrict__ wcn, const double* __restrict__ dtgp, double* __restrict__ hp,
-    double* __restrict__ kx, double* __restrict__ ky, double* __restrict__ kzf,
-    double* __restrict__ qx, double* __restrict__ qy, double* __restrict__ qzf,
-    double* __restrict__ wcu, uint8_t* __restrict__ satf, int* __restrict__ colflag,
-    double* __restrict__ partial) {
-  correct_body<E>(d, f, x, hn, wcn, dtgp, hp, kx, ky, kzf, qx, qy, qzf, wcu, satf, colflag,
-                  partial);
 }
 
 // ---------------------------------------------------------------- post-allocation
@@ -2676,52 +2242,6 @@ void launch_assemble(const Device& D, const double* hn, const double* wcn, bool 
                                                      D.rhs, warm ? D.x : nullptr,
                                                      warm ? hprev : nullptr, ratio);
   D.launches += 2;
-}
-
-// The fused predictor where it applies (groundwater-only domain, nz <= 256);
-// false: the caller launches the separate passes.
-bool launch_predict(const Device& D, const double* hn, const double* wcn, bool mixed) {
-  if (D.f.cpl != nullptr || D.f.baro != nullptr || D.d.nz > 256) return false;
-  const int E = D.d.nz <= 32 ? 1 : D.d.nz <= 64 ? 2 : D.d.nz <= 128 ? 4 : 8;
-  using Kern = void (*)(Dims, Fields, const double*, const double*, const double*, double*,
-                        double*, double*, double*, double*, double*, float*, float*, float*,
-                        float*, float*, float*);
-  Kern k;
-  if (mixed) k = E == 1 ? k_predict<1, true> : E == 2 ? k_predict<2, true>
-               : E == 4 ? k_predict<4, true> : k_predict<8, true>;
-  else k = E == 1 ? k_predict<1, false> : E == 2 ? k_predict<2, false>
-         : E == 4 ? k_predict<4, false> : k_predict<8, false>;
-  const size_t smem = pred_smem_bytes(E);
-  if (raise_smem_limit(reinterpret_cast<const void*>(k), smem) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  const dim3 grid((D.d.nx + kPredCols - 1) / kPredCols, (D.d.ny + kPredRows - 1) / kPredRows);
-  k<<<grid, kPredWarps * 32, smem, D.stream>>>(D.d, D.f, hn, wcn, dtg_slot(D), D.diag, D.gxp,
-                                                D.gyp, D.gzp, D.rhs, mixed ? D.x : nullptr,
-                                                D.diag32, D.gxp32, D.gyp32, D.gzp32, D.dinv32,
-                                                D.l32);
-  ++D.launches;
-  return true;
-}
-
-// The fused corrector where it applies (groundwater-only domain, nz <= 256);
-// false: the caller launches the separate passes.
-bool launch_correct(const Device& D, const double* hn, const double* wcn) {
-  if (D.f.cpl != nullptr || D.f.baro != nullptr || D.d.nz > 256) return false;
-  const int E = D.d.nz <= 32 ? 1 : D.d.nz <= 64 ? 2 : D.d.nz <= 128 ? 4 : 8;
-  const auto k = E == 1 ? k_correct<1> : E == 2 ? k_correct<2> : E == 4 ? k_correct<4>
-                                                                  : k_correct<8>;
-  const size_t smem = corr_smem_bytes(E);
-  if (raise_smem_limit(reinterpret_cast<const void*>(k), smem) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  k<<<cells_grid(D), kCorrWarps * 32, smem, D.stream>>>(
-      D.d, D.f, D.x, hn, wcn, dtg_slot(D), D.hp, D.kx, D.ky, D.kzf, D.qx, D.qy, D.qzf, D.wcu,
-      D.satf, D.colflag, D.partial + kPSs * D.nblk);
-  ++D.launches;
-  return true;
 }
 
 void launch_closure_corr(const Device& D, const double* hn) {
