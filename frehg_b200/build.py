@@ -17,7 +17,7 @@ SOURCES = ["gw_api.cu", "gw_kernels.cu", "gw_cg.cu", "gw_cg_mixed.cu", "gw_cg_li
            "gw_couple.cu", "gw_density.cu",
            "gw_setup.cpp"]
 HEADERS = ["gw_device.cuh", "gw_internal.h", "gw_setup.h", "gw_coop.cuh", "gw_handle.h",
-           "gw_linefactor.cuh", "gw_linesolve.cuh"]
+           "gw_linefactor.cuh", "gw_linesolve.cuh", "gw_cg_line.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

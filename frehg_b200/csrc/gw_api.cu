@@ -18,6 +18,7 @@
 #include "gw_setup.h"
 
 #include "gw_handle.h"
+#include "gw_linesolve.cuh"
 
 namespace {
 thread_local std::string g_error;
@@ -196,31 +197,40 @@ int frehg_gw_create(const frehg_gw_desc* desc, frehg_gw_handle** out) {
       if (e == cudaSuccess) e = dalloc(D, &D.qzf, nf);
       if (e == cudaSuccess) e = dalloc(D, &D.colflag, d.ncol);
       if (e == cudaSuccess) e = dalloc(D, &D.satf, n3);
-      double** solv[] = {&D.diag, &D.gxp, &D.gyp, &D.gzp, &D.rhs, &D.x, &D.r, &D.z, &D.p0, &D.p1, &D.w};
+      // Line solves' columns are padded to a multiple of four cells.
+      const long long np = d.ncol * fgw::line_nzp(d.nz);
+      const long long mp = static_cast<long long>(d.nx2) * fgw::line_nzp(d.nz);
+      const bool line64 = desc->precision == FREHG_GW_PRECISION_FP64_LINE;
+      double** solv[] = {&D.diag, &D.gxp, &D.gyp, &D.gzp, &D.rhs, &D.x};
       for (double** p : solv)
         if (e == cudaSuccess) e = dalloc_margin(D, p, n3, m);
+      double** vecs[] = {&D.r, &D.z, &D.p0, &D.p1, &D.w};
+      for (double** p : vecs)
+        if (e == cudaSuccess) e = line64 ? dalloc_margin(D, p, np, mp) : dalloc_margin(D, p, n3, m);
       if (desc->precision == FREHG_GW_PRECISION_MIXED) {
-        float** solv32[] = {&D.diag32, &D.gxp32, &D.gyp32, &D.gzp32, &D.dinv32, &D.l32,
-                            &D.r32,    &D.z32,   &D.d32,   &D.p032,  &D.p132, &D.w32};
-        for (float** p : solv32)
-          if (e == cudaSuccess) e = dalloc_margin(D, p, n3, m);
+        fgw::LineVecs<float>& v = D.line32;
+        float** arr[] = {&v.s, &v.l, &v.gx, &v.gy, &v.r, &v.z, &v.p0, &v.p1, &v.w, &v.d};
+        for (float** p : arr)
+          if (e == cudaSuccess) e = dalloc_margin(D, p, np, mp);
+      }
+      if (line64) {
+        fgw::LineVecs<double>& v = D.line64;
+        double** arr[] = {&v.s, &v.l, &v.gx, &v.gy, &v.d};
+        for (double** p : arr)
+          if (e == cudaSuccess) e = dalloc_margin(D, p, np, mp);
+        v.r = D.r;
+        v.z = D.z;
+        v.p0 = D.p0;
+        v.p1 = D.p1;
+        v.w = D.w;
+      }
+      if (line64 || desc->precision == FREHG_GW_PRECISION_MIXED)
         if (e == cudaSuccess) e = dalloc_margin(D, &D.xalt, n3, m);
-      }
-      if (desc->precision == FREHG_GW_PRECISION_FP64_LINE) {
-        double** line64[] = {&D.dinv64, &D.l64, &D.d64, &D.xalt};
-        for (double** p : line64)
-          if (e == cudaSuccess) e = dalloc_margin(D, p, n3, m);
-      }
       // Diagonal 1 everywhere outside the active rows (ghosts, margins), so the
       // Jacobi scaling of those always-zero entries stays finite.
       if (e == cudaSuccess && !D.arena_plan) {
         std::vector<double> ones(static_cast<size_t>(n3 + 2 * m), 1.0);
         e = cudaMemcpy(D.diag - m, ones.data(), ones.size() * sizeof(double), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && D.diag32) {
-          std::vector<float> onesf(ones.size(), 1.0f);
-          e = cudaMemcpy(D.diag32 - m, onesf.data(), onesf.size() * sizeof(float),
-                         cudaMemcpyHostToDevice);
-        }
       }
       D.nblk = static_cast<int>(std::min<long long>((n3 + fgw::kBlock - 1) / fgw::kBlock,
                                                     static_cast<long long>(D.sm_count) * 8));

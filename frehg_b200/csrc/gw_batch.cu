@@ -126,6 +126,8 @@ size_t args_bytes(const SolveClass& c) {
   return c.kind == 0 ? cg64_args_bytes() : mixed_args_bytes();
 }
 
+int batch_block(const SolveClass& c) { return c.kind == 0 ? coop::kCgBlock : line_block(); }
+
 const void* batch_kernel(const SolveClass& c) {
   return c.kind == 0 ? cg64_batch_kernel() : mixed_batch_kernel();
 }
@@ -137,11 +139,10 @@ SolveClass solve_class(const Device& D, int precision, bool tiled_line_solve) {
   return SolveClass{0, (D.d.nz % 2 == 0) ? 1 : 0};
 }
 
-int solve_blocks_per_sm(const SolveClass& c, size_t smem) {
+int solve_blocks_per_sm(const SolveClass& c) {
   const void* k = batch_kernel(c);
-  if (smem > 0) raise_smem_limit(k, smem);
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, coop::kCgBlock, smem) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, batch_block(c), 0) !=
       cudaSuccess)
     per_sm = 0;
   return per_sm;
@@ -171,14 +172,12 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   std::vector<int> first(ds.size() + 1, 0);
   std::vector<CgState*> st(ds.size());
   std::vector<double*> parts(ds.size());
-  g.smem = 0;
   for (size_t i = 0; i < ds.size(); ++i) {
     if (c.kind == 0) cg64_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
     else mixed_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
     first[i + 1] = first[i] + nb[i];
     st[i] = &ds[i]->out->cg;
     parts[i] = ds[i]->cgpart;
-    if (c.kind == 1) g.smem = std::max(g.smem, mixed_batch_smem(*ds[i], variants[i]));
   }
   g.slots = first.back();
   g.grid = std::min(g.slots, max_grid);
@@ -201,8 +200,6 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
     e = cudaMemcpy(g.states, st.data(), st.size() * sizeof(CgState*), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(g.parts, parts.data(), parts.size() * sizeof(double*), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && g.smem > 0)
-    e = raise_smem_limit(batch_kernel(c), g.smem);
   return e;
 }
 
@@ -215,8 +212,8 @@ cudaError_t solve_group_launch(const SolveGroup& g, cudaStream_t s) {
   int* order = g.order;
   int* ofirst = g.ofirst;
   void* args[] = {&tab, &first, &n, &queue, &order, &ofirst};
-  return cudaLaunchCooperativeKernel(batch_kernel(g.cls), dim3(g.grid), dim3(coop::kCgBlock), args,
-                                     g.smem, s);
+  return cudaLaunchCooperativeKernel(batch_kernel(g.cls), dim3(g.grid), dim3(batch_block(g.cls)), args, 0,
+                                     s);
 }
 
 
@@ -288,16 +285,13 @@ int build_groups(frehg_gw_batch* b) {
   };
   std::vector<Spec> specs;
   for (int kind = 0; kind < 2; ++kind) {
-    size_t smem = 0;
     bool any = false;
     for (int j = 0; j < n; ++j) {
-      if (cls[j].kind != kind) continue;
-      any = true;
-      if (kind == 1) smem = std::max(smem, fgw::mixed_batch_smem(b->m[j]->D, cls[j].variant));
+      if (cls[j].kind == kind) any = true;
     }
     if (!any) continue;
     const fgw::SolveClass c{kind, 0};
-    const int per_sm = fgw::solve_blocks_per_sm(c, smem);
+    const int per_sm = fgw::solve_blocks_per_sm(c);
     if (per_sm < 1) return fail(FREHG_GW_ECUDA, "batch: solve kernel cannot be resident");
     Spec cur{c, 0, {}, {}, {}, {}};
     for (int j = 0; j < n; ++j) {

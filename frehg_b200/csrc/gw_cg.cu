@@ -261,7 +261,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   }
   if (tail) cg64_cell_init(a, ct, rr, zz);
   double s2[2] = {zz, rr};
-  if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+  if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st)) return;
   double dp = sqrt(s2[0]);
   double beta = s2[1];
   const double rnorm0 = dp;
@@ -298,7 +298,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       pw = cg64_phase_a<ALIGNED, W, false, false>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
     if (tail) cg64_cell_stencil(a, ct, i == 0, (i & 1) != 0, bc, al, al1, pold, pnew, pw);
     double s1[1] = {pw};
-    if (!grid_sum(s1, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(s1, a.part, bid, G, epoch, a.st)) return;
     dpiold = dpi;
     dpi = s1[0];
     betaold = beta;
@@ -328,7 +328,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     if (tail) cg64_cell_update(a, ct, al, rr, zz);
     s2[0] = zz;
     s2[1] = rr;
-    if (!grid_sum(s2, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st)) return;
     dp = sqrt(s2[0]);
     test(dp);
     if (reason != 0) break;

@@ -48,22 +48,22 @@ __device__ inline double warp_sum(double v) {
   return v;
 }
 
-// Sum of a block's warp sums, pairwise (a chain of 16 additions is 0.15 us).
+// Sum of a block's N warp sums, pairwise (a chain of 16 additions is 0.15 us).
+template <int N>
 __device__ inline double tree_sum(const double* w) {
-  constexpr int kWarps = kCgBlock / 32;
-  double t[kWarps];
+  double t[N];
 #pragma unroll
-  for (int q = 0; q < kWarps; ++q) t[q] = w[q];
+  for (int q = 0; q < N; ++q) t[q] = w[q];
 #pragma unroll
-  for (int m = kWarps / 2; m > 0; m >>= 1) {
+  for (int m = 1; m < N; m <<= 1) {
 #pragma unroll
-    for (int q = 0; q < m; ++q) t[q] += t[q + m];
+    for (int q = 0; q + m < N; q += 2 * m) t[q] += t[q + m];
   }
   return t[0];
 }
 
 // Grid barrier and sum in one exchange, for a cooperative (co-resident)
-// launch of kCgBlock threads a block: v[n] <- the sum of every thread's v[n]
+// launch of BLOCK threads a block: v[n] <- the sum of every thread's v[n]
 // over the G blocks, the same bits in every thread (fixed order: lanes, warps,
 // then blocks by stripes of the block's threads).  Writes made before the call
 // by any thread of the G blocks are visible after it.
@@ -80,11 +80,11 @@ __device__ inline double tree_sum(const double* w) {
 //
 // The wait is bounded: past kSpinLimit polls thread 0 sets CgState::err and
 // every block returns false here or at its next call, and leaves the kernel.
-template <int NV>
+template <int BLOCK, int NV>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const int bid,
                                          const int G, unsigned& epoch, CgState* st) {
   static_assert(NV <= kRedVals, "slots");
-  constexpr int kWarps = kCgBlock / 32;
+  constexpr int kWarps = BLOCK / 32;
   __shared__ double sh[NV][kWarps];
   __shared__ double sw[NV][kWarps];
   __shared__ int good;
@@ -100,7 +100,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
     ++epoch;
     if (wid == 0) {
       if (lane < NV) {
-        const double s = tree_sum(sh[lane]);
+        const double s = tree_sum<kWarps>(sh[lane]);
         st_relaxed_f64(gen + static_cast<long long>(lane) * G + bid, s);
       }
       __syncwarp();
@@ -127,7 +127,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
     if (!good) return false;
 #pragma unroll
     for (int n = 0; n < NV; ++n) v[n] = 0.0;
-    for (int b = threadIdx.x; b < G; b += kCgBlock) {
+    for (int b = threadIdx.x; b < G; b += BLOCK) {
 #pragma unroll
       for (int n = 0; n < NV; ++n) v[n] += ld_relaxed_f64(gen + static_cast<long long>(n) * G + b);
     }
@@ -138,10 +138,10 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
     }
     __syncthreads();
 #pragma unroll
-    for (int n = 0; n < NV; ++n) v[n] = tree_sum(sw[n]);
+    for (int n = 0; n < NV; ++n) v[n] = tree_sum<kWarps>(sw[n]);
   } else {
 #pragma unroll
-    for (int n = 0; n < NV; ++n) v[n] = tree_sum(sh[n]);
+    for (int n = 0; n < NV; ++n) v[n] = tree_sum<kWarps>(sh[n]);
     __syncthreads();
   }
   return true;

@@ -64,6 +64,15 @@ constexpr int kBlock = 256;
 // Reduction slots (doubles) a solve block needs (coop::grid_sum).
 constexpr size_t kSolveSlots = 8;
 
+// Arrays of a line solve in its inner precision, in the padded column layout of
+// gw_linesolve.cuh: the pivots' scaling s, the scaled column factor l and
+// lateral legs gx, gy, and the inner CG vectors.
+template <typename T>
+struct LineVecs {
+  T *s = nullptr, *l = nullptr, *gx = nullptr, *gy = nullptr;
+  T *r = nullptr, *z = nullptr, *p0 = nullptr, *p1 = nullptr, *w = nullptr, *d = nullptr;
+};
+
 struct Device {
   Dims d{};
   Fields f{};
@@ -113,14 +122,12 @@ struct Device {
   // on both ends; the pointers below point at cell 0.
   double *diag = nullptr, *gxp = nullptr, *gyp = nullptr, *gzp = nullptr, *rhs = nullptr;
   double *x = nullptr, *r = nullptr, *z = nullptr, *p0 = nullptr, *p1 = nullptr, *w = nullptr;
-  // mixed precision: FP32 copies and inner vectors (same margins)
-  float *diag32 = nullptr, *gxp32 = nullptr, *gyp32 = nullptr, *gzp32 = nullptr;
-  float *dinv32 = nullptr, *l32 = nullptr;  // LDL^T factors of the column blocks
-  float *r32 = nullptr, *z32 = nullptr, *d32 = nullptr, *p032 = nullptr, *p132 = nullptr,
-        *w32 = nullptr;
-  double* xalt = nullptr;  // FP64 ping-pong partner of x (mixed / FP64 line outer sweeps)
-  // FP64 line form: the column factors in FP64 and the correction d
-  double *dinv64 = nullptr, *l64 = nullptr, *d64 = nullptr;
+  // Line solves (padded columns, one j-row of margin on both ends): FP32 for
+  // the mixed form, FP64 for the FP64 line form (whose r, z, p, w are the
+  // arrays above)
+  LineVecs<float> line32;
+  LineVecs<double> line64;
+  double* xalt = nullptr;  // FP64 ping-pong partner of x (line solves' outer sweeps)
   // reductions
   double* partial = nullptr;   // kPSlots x nblk
   double* cgpart = nullptr;    // coop::kRedSlots x cg grid: the solves' reduction slots
@@ -170,8 +177,8 @@ void launch_init_state(const Device& D, int form, double constant, const double*
 // FP64 Jacobi-PCG (PETSc KSPCG semantics); returns a CUDA error code.
 cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit);
 // FP32-inner / FP64-outer defect correction.
-// FP32 casts of the coefficients and the per-column LDL^T factors of the
-// mixed solve's line preconditioner (one launch before launch_cg_mixed).
+// The column factors and scaling of the mixed solve (one launch before
+// launch_cg_mixed).
 cudaError_t launch_line_factor(Device& D);
 cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, double outer_rtol,
                             int max_outer);
@@ -199,13 +206,13 @@ struct alignas(16) StepArgs {
   double *hp, *wcu, *ch, *kcx, *kcy, *kcz, *kx, *ky, *kzf, *qx, *qy, *qzf;
   double *vloss, *room, *sup, *sdn;
   double *diag, *gxp, *gyp, *gzp, *rhs, *x;
-  float *diag32, *gxp32, *gyp32, *gzp32, *dinv32, *l32;
+  float *s32, *l32;
   uint8_t* satf;
   int* colflag;
   double* partial;
   StepOut* out;
   double dtg, co_max, dq_grow, dq_shrink, dt_min, dt_max;
-  int nblk, tc, mixed, warp_walk;
+  int nblk, mixed, warp_walk;
 };
 
 // Device tables of a batch's members for the batched phases.
@@ -215,7 +222,7 @@ struct PhaseTables {
   StepArgs* tab_host = nullptr;  // pinned, refreshed before each step
   int *first_cells = nullptr, *first_ghost = nullptr, *first_factor = nullptr;  // device, n + 1
   int grid_cells = 0, grid_ghost = 0, grid_factor = 0;
-  size_t walk_smem = 0, factor_smem = 0;
+  size_t walk_smem = 0;
   StepOut* outs = nullptr;       // device, n step records gathered
   StepOut* outs_host = nullptr;  // pinned
   int cap = 0;                   // members the buffers hold (reused while n <= cap)
@@ -234,9 +241,9 @@ cudaError_t batch_predictor(const PhaseTables& t, cudaStream_t s);
 cudaError_t batch_corrector(const PhaseTables& t, cudaStream_t s);
 // Launch geometry shared by the single-domain and batched launches.
 int ghost_blocks(const Device& D);
-int line_tile_cols(int nz);
+int line_block();  // threads of a line solve's block
+int line_grid(const Device& D, int variant);
 int line_factor_blocks(const Device& D);
-size_t line_factor_smem(int nz);
 cudaError_t launch_line_factor_batch(const PhaseTables& t, cudaStream_t s);
 
 // ---------------------------------------------------------------- batched solves
@@ -249,14 +256,14 @@ struct SolveParams {
 };
 
 // Kernel variant of a domain's solve: FP64 (kind 0; variant 1 = two cells a
-// thread, nz even) or mixed (kind 1; variant = V * 16 + E, see gw_cg_mixed.cu).
+// thread, nz even) or mixed (kind 1; variant = line_variant, or kLineDeep).
 struct SolveClass {
   int kind, variant;
   bool operator==(const SolveClass& o) const { return kind == o.kind && variant == o.variant; }
 };
 SolveClass solve_class(const Device& D, int precision, bool tiled_line_solve);
 // Blocks of that variant one SM holds (the cooperative limit per SM).
-int solve_blocks_per_sm(const SolveClass& c, size_t smem);
+int solve_blocks_per_sm(const SolveClass& c);
 // Largest block count a member may take (its reduction buffer's capacity).
 int solve_max_blocks(const Device& D, const SolveClass& c);
 
@@ -264,7 +271,6 @@ struct SolveGroup {
   SolveClass cls{0, 0};
   int n = 0, grid = 0;
   int slots = 0;                 // the members' blocks in total (first[n])
-  size_t smem = 0;
   void* tab = nullptr;           // device table of per-member kernel arguments
   int* first = nullptr;          // device block offsets, n + 1
   CgState** states = nullptr;    // device array of the members' CG states
@@ -297,7 +303,6 @@ const void* cg64_batch_kernel();
 int mixed_variant(const Device& D, bool tiled);
 size_t mixed_args_bytes();
 void mixed_fill_args(const Device& D, const SolveParams& p, int variant, void* dst);
-size_t mixed_batch_smem(const Device& D, int variant);
 const void* mixed_batch_kernel();
 
 }  // namespace fgw

@@ -2434,12 +2434,8 @@ void fill_step_args(const Device& D, bool mixed, double dtg, double co_max, doub
   a.gzp = D.gzp;
   a.rhs = D.rhs;
   a.x = D.x;
-  a.diag32 = D.diag32;
-  a.gxp32 = D.gxp32;
-  a.gyp32 = D.gyp32;
-  a.gzp32 = D.gzp32;
-  a.dinv32 = D.dinv32;
-  a.l32 = D.l32;
+  a.s32 = D.line32.s;
+  a.l32 = D.line32.l;
   a.satf = D.satf;
   a.colflag = D.colflag;
   a.partial = D.partial;
@@ -2451,7 +2447,6 @@ void fill_step_args(const Device& D, bool mixed, double dtg, double co_max, doub
   a.dt_min = dt_min;
   a.dt_max = dt_max;
   a.nblk = batch_cell_blocks(D);
-  a.tc = line_tile_cols(D.d.nz);
   a.mixed = mixed ? 1 : 0;
   const size_t smem = kWalkWarps * walk_warp_bytes(D.d.nz);
   a.warp_walk = (D.d.nz <= kWalkMaxNz && smem <= kWalkSmemMax) ? 1 : 0;
@@ -2477,7 +2472,6 @@ cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>&
   }
   std::vector<int> fc(t.n + 1, 0), fg(t.n + 1, 0), ff(t.n + 1, 0);
   t.walk_smem = 0;
-  t.factor_smem = 0;
   for (int i = 0; i < t.n; ++i) {
     const Device& D = *ds[i];
     fc[i + 1] = fc[i] + batch_cell_blocks(D);
@@ -2485,7 +2479,6 @@ cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>&
     ff[i + 1] = ff[i] + (mixed[i] ? line_factor_blocks(D) : 0);
     const size_t ws = kWalkWarps * walk_warp_bytes(D.d.nz);
     if (D.d.nz <= kWalkMaxNz && ws <= kWalkSmemMax) t.walk_smem = std::max(t.walk_smem, ws);
-    if (mixed[i]) t.factor_smem = std::max(t.factor_smem, line_factor_smem(D.d.nz));
   }
   t.grid_cells = fc.back();
   t.grid_ghost = fg.back();

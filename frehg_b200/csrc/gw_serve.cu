@@ -263,9 +263,12 @@ size_t frehg_gw_device_bytes(const frehg_gw_desc* d) {
   b += 14 * r(8 * n3);                      // closures, fluxes, walk scratch
   b += 2 * r(8 * nf);                       // z-face conductivity and flux
   b += r(4 * ncol);                         // column flags
-  b += 11 * r(8 * ns);                      // FP64 solver vectors with margins
-  if (d->precision == FREHG_GW_PRECISION_MIXED) b += 12 * r(4 * ns) + r(8 * ns);
-  if (d->precision == FREHG_GW_PRECISION_FP64_LINE) b += 4 * r(8 * ns);
+  // FP64 solver vectors with margins; the line solves' with padded columns
+  const size_t np = (ncol + 2 * static_cast<size_t>(d->nx + 2)) * ((d->nz + 3) & ~3);
+  const bool line64 = d->precision == FREHG_GW_PRECISION_FP64_LINE;
+  b += 6 * r(8 * ns) + 5 * r(8 * (line64 ? np : ns));
+  if (d->precision == FREHG_GW_PRECISION_MIXED) b += 10 * r(4 * np) + r(8 * ns);
+  if (line64) b += 5 * r(8 * np) + r(8 * ns);
   const size_t nblk = std::min<size_t>((n3 + 255) / 256, 512 * 8);
   const size_t cg = std::max<size_t>((n3 + 255) / 256, 512 * 4);
   b += r(8 * fgw::kPSlots * nblk) + r(8 * fgw::kSolveSlots * cg) + r(sizeof(fgw::StepOut));
