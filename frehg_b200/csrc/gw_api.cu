@@ -11,6 +11,7 @@
 #include <exception>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/frehg_gw.h"
@@ -74,6 +75,116 @@ cudaError_t dalloc_margin(fgw::Device& D, T** p, long long ncell, long long marg
   cudaError_t e = dalloc(D, &base, static_cast<size_t>(ncell + 2 * margin));
   *p = base ? base + margin : nullptr;
   return e;
+}
+
+// Page-locked staging for large field reads, one for the process: two chunks
+// for each copying thread, allocated by the first large read and given back
+// with the last handle.  A read that finds it taken copies without it.
+constexpr int kFetchThreads = 4;
+constexpr size_t kFetchChunk = 2u << 20;
+constexpr size_t kFetchDirect = 8u << 20;  // smaller reads: one plain copy
+
+class FetchStaging {
+ public:
+  void add_handle() {
+    std::lock_guard<std::mutex> lock(mu_);
+    ++handles_;
+  }
+  void drop_handle() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (--handles_ == 0 && mem_ && !taken_) {
+      cudaFreeHost(mem_);
+      mem_ = nullptr;
+    }
+  }
+  char* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (taken_) return nullptr;
+    if (!mem_ && cudaHostAlloc(&mem_, 2 * kFetchThreads * kFetchChunk, cudaHostAllocPortable) !=
+                     cudaSuccess) {
+      cudaGetLastError();
+      mem_ = nullptr;
+      return nullptr;
+    }
+    taken_ = true;
+    return static_cast<char*>(mem_);
+  }
+  void give_back() {
+    std::lock_guard<std::mutex> lock(mu_);
+    taken_ = false;
+    if (handles_ == 0) {
+      cudaFreeHost(mem_);
+      mem_ = nullptr;
+    }
+  }
+
+ private:
+  std::mutex mu_;
+  void* mem_ = nullptr;
+  bool taken_ = false;
+  int handles_ = 0;
+};
+FetchStaging g_fetch;
+
+// Bytes [lo, hi) of src (device) to dst (host) through this thread's two
+// staging chunks: one fills while the other is copied out.
+cudaError_t fetch_range(int device, char* dst, const char* src, size_t lo, size_t hi, char* stage) {
+  cudaError_t e = cudaSetDevice(device);
+  cudaStream_t st = nullptr;
+  cudaEvent_t done[2] = {};
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  for (cudaEvent_t& ev : done)
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  const size_t chunks = (hi - lo + kFetchChunk - 1) / kFetchChunk;
+  const auto size = [&](size_t c) { return std::min(kFetchChunk, hi - lo - c * kFetchChunk); };
+  for (size_t c = 0; c <= chunks && e == cudaSuccess; ++c) {
+    if (c < chunks) {
+      e = cudaMemcpyAsync(stage + (c & 1) * kFetchChunk, src + lo + c * kFetchChunk, size(c),
+                          cudaMemcpyDeviceToHost, st);
+      if (e == cudaSuccess) e = cudaEventRecord(done[c & 1], st);
+    }
+    if (c > 0 && e == cudaSuccess) {
+      e = cudaEventSynchronize(done[(c - 1) & 1]);
+      if (e == cudaSuccess)
+        std::memcpy(dst + lo + (c - 1) * kFetchChunk, stage + ((c - 1) & 1) * kFetchChunk,
+                    size(c - 1));
+    }
+  }
+  if (st) cudaStreamSynchronize(st);  // the staging is free when this returns
+  for (cudaEvent_t ev : done)
+    if (ev) cudaEventDestroy(ev);
+  if (st) cudaStreamDestroy(st);
+  return e;
+}
+
+// Device to host, large copies by kFetchThreads threads at once (the host
+// side, first touches of the caller's pages above all, is what a large read
+// spends its time on).  The source must be complete.
+cudaError_t fetch(int device, double* dst, const double* src, size_t n) {
+  const size_t bytes = n * sizeof(double);
+  char* const stage = bytes > kFetchDirect ? g_fetch.take() : nullptr;
+  if (!stage) return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+  char* const d = reinterpret_cast<char*>(dst);
+  const char* const s = reinterpret_cast<const char*>(src);
+  const size_t part = (bytes / kFetchThreads + 4095) & ~static_cast<size_t>(4095);
+  cudaError_t err[kFetchThreads] = {};
+  const auto range = [&](int t) {
+    const size_t lo = std::min(bytes, t * part), hi = std::min(bytes, lo + part);
+    if (lo < hi) err[t] = fetch_range(device, d, s, lo, hi, stage + 2 * t * kFetchChunk);
+  };
+  std::thread threads[kFetchThreads];
+  int started = 1;
+  try {
+    for (; started < kFetchThreads; ++started) threads[started] = std::thread(range, started);
+  } catch (const std::exception&) {  // no more threads: the caller takes the rest
+  }
+  range(0);
+  for (int t = started; t < kFetchThreads; ++t) range(t);
+  for (int t = 1; t < started; ++t) threads[t].join();
+  g_fetch.give_back();
+  for (cudaError_t e : err)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
 }
 
 void free_device(fgw::Device& D) {
@@ -312,6 +423,7 @@ int frehg_gw_create(const frehg_gw_desc* desc, frehg_gw_handle** out) {
     hnd->co_max = desc->courant_max;
     hnd->next_dt = desc->dt_init;
     CUDA_TRY(cudaDeviceSynchronize(), "frehg_gw_create");
+    g_fetch.add_handle();
     *out = hnd;
     return FREHG_GW_OK;
   } catch (const std::exception& ex) {
@@ -328,6 +440,7 @@ int frehg_gw_destroy(frehg_gw_handle* h) {
   if (h->values_pinned) cudaHostUnregister(h->values.data());
   free_device(h->D);
   delete h;
+  g_fetch.drop_handle();
   return FREHG_GW_OK;
 }
 
@@ -746,21 +859,25 @@ int frehg_gw_get_field(frehg_gw_handle* h, int field, double* out) {
       for (int i = 1; i <= d.nx; ++i) out[q++] = full[fgw::col2(d, j, i)];
     return FREHG_GW_OK;
   }
-  const size_t n = static_cast<size_t>(kind == 3 ? d.ncol * (d.nz + 1) : d.ncell);
-  std::vector<double> full(n);
-  CUDA_TRY(cudaStreamSynchronize(D.stream), "get_field");
-  CUDA_TRY(cudaMemcpy(full.data(), src, n * sizeof(double), cudaMemcpyDeviceToHost), "get_field");
-  size_t q = 0;
-  if (kind == 3) {
-    for (int j = 1; j <= d.ny; ++j)
-      for (int i = 1; i <= d.nx; ++i)
-        for (int k = 0; k <= d.nz; ++k) out[q++] = full[fgw::fidx(d, j, i, k)];
+  // The owned part is packed on the device into a solve vector (scratch
+  // between steps) and read back as one run.  A z-face field of a very flat
+  // domain can exceed it and is read whole.
+  const size_t count = frehg_gw_field_size(h, field);
+  if (count <= static_cast<size_t>(d.ncell)) {
+    fgw::launch_pack(D, src, kind, D.w);
+    CUDA_TRY(cudaGetLastError(), "get_field");
+    CUDA_TRY(cudaStreamSynchronize(D.stream), "get_field");
+    CUDA_TRY(fetch(h->device, out, D.w, count), "get_field");
     return FREHG_GW_OK;
   }
-  const int j0 = (kind == 2) ? 0 : 1, i0 = (kind == 1) ? 0 : 1;
-  for (int j = j0; j <= d.ny; ++j)
-    for (int i = i0; i <= d.nx; ++i)
-      for (int k = 0; k < d.nz; ++k) out[q++] = full[fgw::cidx(d, j, i, k)];
+  std::vector<double> full(static_cast<size_t>(d.ncol) * (d.nz + 1));
+  CUDA_TRY(cudaStreamSynchronize(D.stream), "get_field");
+  CUDA_TRY(cudaMemcpy(full.data(), src, full.size() * sizeof(double), cudaMemcpyDeviceToHost),
+           "get_field");
+  size_t q = 0;
+  for (int j = 1; j <= d.ny; ++j)
+    for (int i = 1; i <= d.nx; ++i)
+      for (int k = 0; k <= d.nz; ++k) out[q++] = full[fgw::fidx(d, j, i, k)];
   return FREHG_GW_OK;
 }
 

@@ -162,6 +162,9 @@ void launch_finalize(const Device& D, double* wc_out, double co_max);
 void launch_step_info(const Device& D, double dq_grow, double dq_shrink, double dt_min,
                       double dt_max);
 void launch_volume(const Device& D, const double* wc);
+// The owned cells (kind 0), x / y faces (1, 2) or z faces (3) of a field, packed
+// in (j, i, k) order into out.
+void launch_pack(const Device& D, const double* field, int kind, double* out);
 // Density coupling: the cell and face ratios from the attached scalars.
 void launch_baro(const Device& D);
 // Coupled top: exchange modes (before the predictor), bookkeeping (after the

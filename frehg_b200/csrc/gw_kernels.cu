@@ -1928,6 +1928,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_finalize(Dims d, Fields f, double
   finalize_body(d, f, wc, vloss, qx, qy, qzf, dtgp, co_max, partial, nblk, blockIdx.x, gridDim.x);
 }
 
+// A warp a column (nzf consecutive values), columns (j0.., i0..) of the halo
+// layout to the packed one.  Bound by HBM and, in the caller, by the read-back.
+__global__ void k_pack(Dims d, const double* __restrict__ field, int nzf, int j0, int i0, int ni,
+                       int n, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+  for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < n; c += warps) {
+    const int j = c / ni, i = c - j * ni;
+    const double* src = field + col2(d, j0 + j, i0 + i) * nzf;
+    double* dst = out + static_cast<long long>(c) * nzf;
+    for (int k = lane; k < nzf; k += 32) dst[k] = src[k];
+  }
+}
+
 __global__ void k_volume(Dims d, Fields f, const double* __restrict__ wc, double* partial) {
   double vol = 0.0;
   for (long long c = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; c < d.ncell;
@@ -2215,6 +2228,15 @@ inline const double* dtg_slot(const Device& D) { return &D.out->next_dt; }
 int ghost_blocks(const Device& D) {
   const long long n = 2LL * (D.d.nx + D.d.ny) * D.d.nz;
   return static_cast<int>(std::min<long long>((n + kBlock - 1) / kBlock, 4096));
+}
+
+void launch_pack(const Device& D, const double* field, int kind, double* out) {
+  const int j0 = kind == 2 ? 0 : 1, i0 = kind == 1 ? 0 : 1;
+  const int ni = D.d.nx + 1 - i0, n = (D.d.ny + 1 - j0) * ni;
+  const int blocks = std::min((n + kBlock / 32 - 1) / (kBlock / 32), 16 * D.sm_count);
+  k_pack<<<blocks, kBlock, 0, D.stream>>>(D.d, field, kind == 3 ? D.d.nz + 1 : D.d.nz, j0, i0, ni,
+                                          n, out);
+  ++D.launches;
 }
 
 void launch_ghosts(const Device& D, double* h, double* wc) {
