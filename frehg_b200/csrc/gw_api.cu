@@ -352,6 +352,7 @@ int frehg_gw_create(const frehg_gw_desc* desc, frehg_gw_handle** out) {
         e = dalloc(D, &D.partial, static_cast<size_t>(fgw::kPSlots) * D.nblk);
       if (e == cudaSuccess)
         e = dalloc(D, &D.cgpart, fgw::kSolveSlots * static_cast<size_t>(std::max(D.cg_grid, D.cg_grid32)));
+      if (e == cudaSuccess) e = dalloc(D, &D.small_sync, fgw::kSmallSyncWords);
       if (e == cudaSuccess) e = dalloc(D, &D.out, 1);
       return e;
     };
@@ -727,30 +728,50 @@ int frehg_gw_step(frehg_gw_handle* h, double t, double dtg, frehg_gw_step_info* 
   auto mark = [&](int n) {
     if (prof) cudaEventRecord(h->ev[n], D.stream);
   };
-  // The step's dtg goes into the device step record, where every kernel of
-  // the step reads it.
-  D.out_host->next_dt = dtg;
-  CUDA_TRY(cudaMemcpyAsync(&D.out->next_dt, &D.out_host->next_dt, sizeof(double),
-                           cudaMemcpyHostToDevice, D.stream), "step dtg");
-  mark(0);
-  cudaError_t e = fgw_api::enqueue_predictor(h, dtg);
+  const bool mixed = h->precision == FREHG_GW_PRECISION_MIXED;
+  const bool line64 = h->precision == FREHG_GW_PRECISION_FP64_LINE;
+  // Small domains run the phases around the solve as one launch each; with
+  // profiling on, which times the phases apart, they run separately.
+  const bool small = !prof && fgw::small_domain(D);
+  cudaError_t e = cudaSuccess;
+  if (small) {
+    D.out_host->cg.err = 1;  // until k_small_post has written the record
+    const bool extrap = (mixed || line64) && h->extrapolate && h->have_prev && h->prev_dtg > 0.0;
+    e = fgw::launch_small_pre(D, mixed, mixed || line64, dtg, extrap ? D.h[1 - D.cur] : nullptr,
+                              extrap ? dtg / h->prev_dtg : 0.0);
+    if (e == cudaSuccess && line64) e = fgw::launch_line_factor64(D);
+  } else {
+    // The step's dtg goes into the device step record, where every kernel of
+    // the step reads it.
+    D.out_host->next_dt = dtg;
+    CUDA_TRY(cudaMemcpyAsync(&D.out->next_dt, &D.out_host->next_dt, sizeof(double),
+                             cudaMemcpyHostToDevice, D.stream), "step dtg");
+    mark(0);
+    e = fgw_api::enqueue_predictor(h, dtg);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "predictor launch");
   mark(1);
-  if (h->precision == FREHG_GW_PRECISION_MIXED) {
-    e = fgw::launch_cg_mixed(D, h->rtol, h->atol, h->maxit, h->outer_rtol, h->max_outer);
-  } else if (h->precision == FREHG_GW_PRECISION_FP64_LINE) {
-    e = fgw::launch_cg_line64(D, h->atol, h->maxit, h->outer_rtol, h->max_outer);
+  if (mixed) {
+    e = fgw::launch_cg_mixed(D, h->rtol, h->atol, h->maxit, h->outer_rtol, h->max_outer, !small);
+  } else if (line64) {
+    e = fgw::launch_cg_line64(D, h->atol, h->maxit, h->outer_rtol, h->max_outer, !small);
   } else {
-    e = fgw::launch_cg64(D, h->rtol, h->atol, h->maxit);
+    e = fgw::launch_cg64(D, h->rtol, h->atol, h->maxit, !small);
   }
   if (e != cudaSuccess) return cuda_fail(e, "predictor solve launch");
   mark(2);
-  fgw_api::enqueue_corrector(h);
-  mark(5);
-  CUDA_TRY(cudaMemcpyAsync(D.out_host, D.out, sizeof(fgw::StepOut), cudaMemcpyDeviceToHost,
-                           D.stream), "step readback");
+  if (small) {
+    e = fgw::launch_small_post(D, h->co_max, h->dq_grow, h->dq_shrink, h->dt_min, h->dt_max);
+    if (e != cudaSuccess) return cuda_fail(e, "corrector launch");
+  } else {
+    fgw_api::enqueue_corrector(h);
+    mark(5);
+    CUDA_TRY(cudaMemcpyAsync(D.out_host, D.out, sizeof(fgw::StepOut), cudaMemcpyDeviceToHost,
+                             D.stream), "step readback");
+  }
   CUDA_TRY(cudaStreamSynchronize(D.stream), "step");
   CUDA_TRY(cudaGetLastError(), "step kernels");
+  if (small && D.out_host->cg.err) fgw::reset_small_sync(D);
   if (prof) {
     for (int n = 0; n < 5; ++n) {
       float ms = 0.0f;

@@ -468,8 +468,8 @@ Cg64Kernel cg64_kernel(int w) {
 
 }  // namespace
 
-cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit) {
-  cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool clear) {
+  if (clear) cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
   Cg64Args a = make_cg64_args(D, rtol, atol, maxit);
   const long long threads = static_cast<long long>(D.cg_grid) * kCgBlock;
   const long long pairs = std::max<long long>(1, (D.d.ncell / 2 + threads - 1) / threads);

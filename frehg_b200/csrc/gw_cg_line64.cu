@@ -48,7 +48,7 @@ cudaError_t launch_line_factor64(Device& D) {
 }
 
 cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rtol,
-                             int max_outer) {
+                             int max_outer, bool clear) {
   const int variant = line_variant(D.d.nz);
   if (variant == kLineDeep) return cudaErrorInvalidValue;
   const int G = line_grid(D, variant);
@@ -62,7 +62,7 @@ cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rto
   const size_t smem = sizeof(Quad<double>) * kLineBlock * static_cast<size_t>(w) * per;
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
-  cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+  if (clear) cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
   LineArgs<double> a;
   a.d = D.d;
   a.diag = D.diag;

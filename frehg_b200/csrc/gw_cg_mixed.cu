@@ -127,7 +127,7 @@ cudaError_t launch_line_factor(Device& D) {
 }
 
 cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, double outer_rtol,
-                            int max_outer) {
+                            int max_outer, bool clear) {
   (void)rtol;
   if (D.d.nz > kMixedMaxNz) return cudaErrorInvalidValue;
   const int variant = line_variant(D.d.nz), G = line_grid(D, variant);
@@ -143,7 +143,7 @@ cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, doub
   const size_t smem = sizeof(Quad<float>) * kLineBlock * static_cast<size_t>(w) * per;
   const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k), smem);
   if (e != cudaSuccess) return e;
-  cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
+  if (clear) cudaMemsetAsync(&D.out->cg, 0, sizeof(CgState), D.stream);
   LineArgs<float> a = make_mixed_args(D, atol, maxit, outer_rtol, max_outer);
   void* args[] = {&a, &per};
   ++D.launches;
@@ -179,13 +179,7 @@ __global__ void __launch_bounds__(kFactorBlock) k_line_factor_batch(const StepAr
     dst[w] = src[w];
   const int bid = blockIdx.x - first[si], G = first[si + 1] - first[si];
   __syncthreads();
-  switch (line_variant(sa.d.nz)) {
-    case 0: line_factor_body<float, 8, 4, false>(sa.d, sa.diag, sa.gzp, sa.s32, sa.l32, bid, G); break;
-    case 1: line_factor_body<float, 16, 4, false>(sa.d, sa.diag, sa.gzp, sa.s32, sa.l32, bid, G); break;
-    case 2: line_factor_body<float, 32, 4, false>(sa.d, sa.diag, sa.gzp, sa.s32, sa.l32, bid, G); break;
-    case 3: line_factor_body<float, 32, 8, false>(sa.d, sa.diag, sa.gzp, sa.s32, sa.l32, bid, G); break;
-    default: line_factor_body<float, 32, 8, true>(sa.d, sa.diag, sa.gzp, sa.s32, sa.l32, bid, G);
-  }
+  line_factor_any(sa, bid, G);
 }
 
 }  // namespace

@@ -48,6 +48,36 @@ __device__ inline double warp_sum(double v) {
   return v;
 }
 
+// Thread 0's part of a grid barrier: counts the block in on `arrived` and polls
+// it up to `want` (which may wrap: the two differ by less than 2^31), with the
+// block's writes released before and the others' acquired after.  Gives up
+// past kSpinLimit polls, or when another block has, by setting *err.
+__device__ inline int arrive_and_wait(unsigned* arrived, unsigned want, int* err) {
+  fence_gpu();
+  red_add(arrived, 1u);
+  int ok = 1;
+  long long spins = 0;
+  while (static_cast<int>(ld_relaxed_u32(arrived) - want) < 0) {
+    ++spins;
+    if (spins > kSpinLimit || ((spins & 1023) == 0 && ld_relaxed_int(err) != 0)) {
+      atomicExch(err, 1);
+      ok = 0;
+      break;
+    }
+  }
+  fence_gpu();
+  return ok;
+}
+
+// Grid barrier without a sum.  False when it gave up; the block then leaves.
+__device__ inline bool grid_barrier(unsigned* arrived, unsigned want, int* err) {
+  __shared__ int good;
+  __syncthreads();
+  if (threadIdx.x == 0) good = arrive_and_wait(arrived, want, err);
+  __syncthreads();
+  return good != 0;
+}
+
 // Sum of a block's N warp sums, pairwise (a chain of 16 additions is 0.15 us).
 template <int N>
 __device__ inline double tree_sum(const double* w) {
@@ -105,22 +135,7 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
       }
       __syncwarp();
       if (lane == 0) {
-        const unsigned want = epoch * static_cast<unsigned>(G);
-        fence_gpu();
-        red_add(&st->arrived, 1u);
-        int ok = 1;
-        long long spins = 0;
-        // arrived - want < 2^31 once all G are in (the difference wraps safely)
-        while (static_cast<int>(ld_relaxed_u32(&st->arrived) - want) < 0) {
-          ++spins;
-          if (spins > kSpinLimit || ((spins & 1023) == 0 && ld_relaxed_int(&st->err) != 0)) {
-            atomicExch(&st->err, 1);
-            ok = 0;
-            break;
-          }
-        }
-        fence_gpu();
-        good = ok;
+        good = arrive_and_wait(&st->arrived, epoch * static_cast<unsigned>(G), &st->err);
       }
     }
     __syncthreads();

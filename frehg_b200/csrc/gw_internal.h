@@ -134,6 +134,8 @@ struct Device {
   int nblk = 0;                // grid of the reducing cell kernels
   int cg_grid = 0;             // co-resident grid of the CG kernel
   int cg_grid32 = 0;
+  unsigned* small_sync = nullptr;   // barrier words of k_small_pre / k_small_post
+  unsigned small_base[2] = {0, 0};  // arrivals counted on them so far
   StepOut* out = nullptr;      // device
   StepOut* out_host = nullptr; // pinned
   std::vector<void*> allocs;   // everything to cudaFree
@@ -178,23 +180,43 @@ void launch_window_accum(const Device& D);
 void launch_init_state(const Device& D, int form, double constant, const double* field,
                        const double* bath, double offset);
 // FP64 Jacobi-PCG (PETSc KSPCG semantics); returns a CUDA error code.
-cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit);
+// clear: zero the CG state first (k_small_pre already has).
+cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool clear = true);
 // FP32-inner / FP64-outer defect correction.
 // The column factors and scaling of the mixed solve (one launch before
 // launch_cg_mixed).
 cudaError_t launch_line_factor(Device& D);
 cudaError_t launch_cg_mixed(Device& D, double rtol, double atol, int maxit, double outer_rtol,
-                            int max_outer);
+                            int max_outer, bool clear = true);
 int cg64_grid(int sm_count, long long ncell);
 // FP64 line form (nz <= 256): FP64 column factors, then the FP64 line-PCG
 // defect-correction solve (the mixed form's algorithm in FP64).
 cudaError_t launch_line_factor64(Device& D);
-cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rtol, int max_outer);
+cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rtol, int max_outer,
+                             bool clear = true);
 
 // Raises (never lowers) a kernel's opt-in dynamic shared-memory limit to
 // `bytes`.  Only raising keeps every launch recorded earlier (in a captured
 // graph, or by another domain) within the limit.
 cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
+
+// ---------------------------------------------------------------- small domains
+// A groundwater-only domain up to kSmallCells cells runs the phases before
+// and after its solve as one cooperative launch each (k_small_pre,
+// k_small_post); the step record lands in D.out_host.  Above, the separate
+// launches' own occupancies win: whole steps, one launch a phase (with its
+// timing events, some 15 us) against two, FP64: 32x32x50 208 -> 153 us,
+// 56x56x80 279 -> 227, 64x64x128 377 -> 345, 80x80x128 482 -> 475,
+// 100x100x100 568 -> 557.
+constexpr long long kSmallCells = 600000;
+constexpr size_t kSmallSyncWords = 64;
+bool small_domain(const Device& D);
+cudaError_t launch_small_pre(Device& D, bool mixed, bool warm, double dtg, const double* hprev,
+                             double ratio);
+cudaError_t launch_small_post(Device& D, double co_max, double dq_grow, double dq_shrink,
+                              double dt_min, double dt_max);
+// After a barrier gave up: the words and their count start over.
+cudaError_t reset_small_sync(Device& D);
 
 // ---------------------------------------------------------------- batched phases
 // One member's arguments for the batched non-solve phases: its geometry and

@@ -80,6 +80,48 @@ __device__ double block_reduce(double v, Op op, double identity) {
   return v;
 }
 
+// Several block reductions at once, each in a fixed order, warp n writing the
+// n-th to its address: the shuffles of all of them overlap and one barrier
+// serves them all (five in turn were 2 us of a small domain's k_finalize).
+// The shared arrays are free again after the block's next barrier.
+enum RedOp { kRedSum, kRedMax, kRedMin };
+struct RedItem {
+  double v;
+  RedOp op;
+  double* out;
+};
+__device__ inline double red_apply(RedOp op, double a, double b) {
+  return op == kRedSum ? a + b : op == kRedMax ? (b > a ? b : a) : (b < a ? b : a);
+}
+__device__ inline double red_identity(RedOp op) {
+  return op == kRedSum ? 0.0 : op == kRedMax ? -DBL_MAX : DBL_MAX;
+}
+__device__ inline double warp_red(RedOp op, double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = red_apply(op, v, __shfl_down_sync(0xffffffffu, v, o));
+  return v;
+}
+template <int N>
+__device__ inline void block_reduce_many(const RedItem (&it)[N]) {
+  constexpr int kWarps = kBlock / 32;
+  static_assert(N <= kWarps, "a warp a value");
+  __shared__ double sh[N][kWarps];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const double v = warp_red(it[n].op, it[n].v);
+    if (lane == 0) sh[n][wid] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    if (wid == n) {
+      const double v = warp_red(it[n].op, lane < kWarps ? sh[n][lane] : red_identity(it[n].op));
+      if (lane == 0) *it[n].out = v;
+    }
+  }
+}
+
 inline dim3 cells_grid(const Device& D) { return dim3(static_cast<unsigned>(D.nblk)); }
 
 // ---------------------------------------------------------------- ghosts
@@ -1112,10 +1154,8 @@ __device__ __forceinline__ void classify_body(
     sup[c] = r.up;
     sdn[c] = r.dn;
   }
-  const double s1 = block_reduce(adj, SumOp(), 0.0);
-  if (threadIdx.x == 0) part_adj[bid] = s1;
-  const double s2 = block_reduce(drop, SumOp(), 0.0);
-  if (threadIdx.x == 0) part_drop[bid] = s2;
+  const RedItem it[2] = {{adj, kRedSum, part_adj + bid}, {drop, kRedSum, part_drop + bid}};
+  block_reduce_many(it);
 }
 
 template <bool BARO>
@@ -1198,13 +1238,14 @@ __device__ inline void vent_store(const Fields& f, long long col, const VentStat
 template <bool CPL>
 __device__ inline void walk_books(const Dims& d, double lost, const VentState& v, double* partial,
                                   int nblk, int bid) {
-  const double s = block_reduce(lost, SumOp(), 0.0);
-  if (threadIdx.x == 0) partial[kPLost * nblk + bid] = s;
-  if (CPL) {
-    const double sv = block_reduce(v.vent, SumOp(), 0.0);
-    if (threadIdx.x == 0) partial[kPVent * nblk + bid] = sv;
-    const double st = block_reduce(v.thin, SumOp(), 0.0);
-    if (threadIdx.x == 0) partial[kPThin * nblk + bid] = st;
+  if constexpr (CPL) {
+    const RedItem it[3] = {{lost, kRedSum, partial + kPLost * nblk + bid},
+                           {v.vent, kRedSum, partial + kPVent * nblk + bid},
+                           {v.thin, kRedSum, partial + kPThin * nblk + bid}};
+    block_reduce_many(it);
+  } else {
+    const RedItem it[1] = {{lost, kRedSum, partial + kPLost * nblk + bid}};
+    block_reduce_many(it);
   }
 }
 
@@ -1863,16 +1904,12 @@ __device__ __forceinline__ double finalize_cell(const Dims& d, const FinIn& v, l
 // The finalize reductions of a block into the partial slots.
 __device__ __forceinline__ void finalize_reduce(const FinAcc& acc, double* partial, int nblk,
                                                 int bid) {
-  double s = block_reduce(acc.vl, SumOp(), 0.0);
-  if (threadIdx.x == 0) partial[kPVloss * nblk + bid] = s;
-  s = block_reduce(acc.inflow, SumOp(), 0.0);
-  if (threadIdx.x == 0) partial[kPInflow * nblk + bid] = s;
-  s = block_reduce(acc.dqmax, MaxOp(), -DBL_MAX);
-  if (threadIdx.x == 0) partial[kPDqmax * nblk + bid] = s;
-  s = block_reduce(acc.dtco, MinOp(), DBL_MAX);
-  if (threadIdx.x == 0) partial[kPDtco * nblk + bid] = s;
-  s = block_reduce(acc.vol, SumOp(), 0.0);
-  if (threadIdx.x == 0) partial[kPVol * nblk + bid] = s;
+  const RedItem it[5] = {{acc.vl, kRedSum, partial + kPVloss * nblk + bid},
+                         {acc.inflow, kRedSum, partial + kPInflow * nblk + bid},
+                         {acc.dqmax, kRedMax, partial + kPDqmax * nblk + bid},
+                         {acc.dtco, kRedMin, partial + kPDtco * nblk + bid},
+                         {acc.vol, kRedSum, partial + kPVol * nblk + bid}};
+  block_reduce_many(it);
 }
 
 __device__ __forceinline__ void finalize_body(Dims d, Fields f, double* __restrict__ wc,
@@ -2008,24 +2045,38 @@ __device__ double reduce_slot(const double* p, int n, Op op, double identity) {
 __device__ __forceinline__ void step_info_body(const double* partial, int nblk, int off, int cpl,
                                                double dq_grow, double dq_shrink, double dt_min,
                                                double dt_max, double dtg, StepOut* out) {
-  const double ss = reduce_slot(partial + kPSs * nblk, nblk, SumOp(), 0.0);
-  const double adj = reduce_slot(partial + kPAdj * nblk, nblk, SumOp(), 0.0);
-  const double drop = reduce_slot(partial + kPDrop * nblk, nblk, SumOp(), 0.0);
-  const double lost = reduce_slot(partial + kPLost * nblk, nblk, SumOp(), 0.0);
-  const double vl = reduce_slot(partial + kPVloss * nblk, nblk, SumOp(), 0.0);
-  const double inflow = reduce_slot(partial + kPInflow * nblk, nblk, SumOp(), 0.0);
-  const double dqmax = reduce_slot(partial + kPDqmax * nblk, nblk, MaxOp(), -DBL_MAX);
-  const double dtco = reduce_slot(partial + kPDtco * nblk, nblk, MinOp(), DBL_MAX);
-  const double vol = reduce_slot(partial + kPVol * nblk, nblk, SumOp(), 0.0);
+  // A warp a slot: all slots' loads are in flight together (nine block
+  // reductions in turn took 10 us).
+  __shared__ double tot[kPSlots];
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int slot = threadIdx.x >> 5; slot < (cpl ? kPSlots : kPExch); slot += warps) {
+    const RedOp op = slot == kPDqmax ? kRedMax : slot == kPDtco ? kRedMin : kRedSum;
+    const double* p = partial + static_cast<long long>(slot) * nblk;
+    double v = red_identity(op);
+    for (int b0 = 0; b0 < nblk; b0 += 32 * 8) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int b = b0 + 32 * u + lane;
+        x[u] = b < nblk ? p[b] : red_identity(op);
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v = red_apply(op, v, x[u]);
+    }
+    v = warp_red(op, v);
+    if (lane == 0) tot[slot] = v;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
-    out->ss_storage = ss;
-    out->realloc_adjust = off ? 0.0 : adj + lost;
-    out->realloc_dropped = off ? 0.0 : drop - lost;
-    out->vloss = vl;
-    out->boundary_in = inflow;
+    const double dqmax = tot[kPDqmax], dtco = tot[kPDtco];
+    out->ss_storage = tot[kPSs];
+    out->realloc_adjust = off ? 0.0 : tot[kPAdj] + tot[kPLost];
+    out->realloc_dropped = off ? 0.0 : tot[kPDrop] - tot[kPLost];
+    out->vloss = tot[kPVloss];
+    out->boundary_in = tot[kPInflow];
     out->dqmax = dqmax;
     out->dtco = dtco;
-    out->volume = vol;
+    out->volume = tot[kPVol];
     double next = dtg;
     if (dqmax > dq_shrink) next = dtg * 0.75;
     else if (dqmax < dq_grow) next = dtg * 1.25;
@@ -2033,15 +2084,15 @@ __device__ __forceinline__ void step_info_body(const double* partial, int nblk, 
     if (next > dt_max) next = dt_max;
     if (next < dt_min) next = dt_min;
     out->next_dt = next;
-  }
-  if (cpl) {
-    // exchanged, bounce, vent, vent_thin, evap, mode-3 clamp (frehg_gw_coupled_audit order);
-    // the reallocation's vent books are zero when it is disabled
-    const int slot[6] = {kPExch, kPBounce, kPVent, kPThin, kPEvap, kPClamp};
-    for (int s = 0; s < 6; ++s) {
-      double v = reduce_slot(partial + slot[s] * nblk, nblk, SumOp(), 0.0);
-      if (off && (slot[s] == kPVent || slot[s] == kPThin)) v = 0.0;
-      if (threadIdx.x == 0) out->cpl[s] = v;
+    if (cpl) {
+      // exchanged, bounce, vent, vent_thin, evap, mode-3 clamp (frehg_gw_coupled_audit order);
+      // the reallocation's vent books are zero when it is disabled
+      out->cpl[0] = tot[kPExch];
+      out->cpl[1] = tot[kPBounce];
+      out->cpl[2] = off ? 0.0 : tot[kPVent];
+      out->cpl[3] = off ? 0.0 : tot[kPThin];
+      out->cpl[4] = tot[kPEvap];
+      out->cpl[5] = tot[kPClamp];
     }
   }
 }
@@ -2200,6 +2251,94 @@ __global__ void k_gather_outs(const StepArgs* tab, StepOut* outs, int n) {
     for (int w = threadIdx.x; w < static_cast<int>(sizeof(StepOut) / 4); w += blockDim.x)
       dst[w] = src[w];
   }
+}
+
+// ---------------------------------------------------------------- small domains
+// The phases before and after the solve in one cooperative launch each, a
+// grid barrier between phases instead of a launch.  A small domain's phases
+// are latency (a few cells a thread), and what a launch costs on top is most
+// of a step: an 8x6x20 step took 91 us in twelve launches, two copies and a
+// memset around its solve, 32 us in these two.  Same bodies, same values; the
+// partial sums' order follows the grid.  Two blocks per SM, so that up to 76k
+// cells every phase is one cell a thread.  The step's dt comes as an argument and the step
+// record goes straight to the host's page-locked copy, so the copies and the
+// memset go too.
+struct SmallArgs {
+  StepArgs a;
+  const double* hprev;
+  double ratio;
+  int warm;
+  unsigned* arrived;  // only grows; the launch's barriers start from base
+  unsigned base;
+  StepOut* host;
+};
+
+__global__ void __launch_bounds__(kBlock, 2) k_small_pre(SmallArgs s) {
+  const StepArgs& a = s.a;
+  const int bid = blockIdx.x, G = gridDim.x;
+  unsigned want = s.base;
+  const auto barrier = [&] {
+    want += G;
+    return G == 1 ? (__syncthreads(), true) : coop::grid_barrier(s.arrived, want, &a.out->cg.err);
+  };
+  if (bid == 0 && threadIdx.x == 0) {
+    a.out->next_dt = a.dtg;
+    a.out->cg = CgState{};
+  }
+  ghosts_body(a.d, a.f, a.hn, a.wcn, bid, G);
+  if (!barrier()) return;
+  closure_pred_body(a.d, a.f, a.hn, a.kcx, a.kcy, a.kcz, a.ch, bid, G);
+  if (!barrier()) return;
+  const PassK pk{a.kcx, a.kcy, a.kcz, a.wcn};
+  faces_body<false>(a.d, a.f, pk, a.kx, a.ky, a.kzf, bid, G);
+  if (!barrier()) return;
+  assemble_body<false, false>(a.d, a.f, a.kx, a.ky, a.kzf, a.hn, a.wcn, a.ch, &a.out->next_dt,
+                              a.diag, a.gxp, a.gyp, a.gzp, a.rhs, s.warm ? a.x : nullptr, s.hprev,
+                              s.ratio, bid, G);
+  if (!a.mixed) return;
+  if (!barrier()) return;
+  line_factor_any(a, bid, G);
+}
+
+__global__ void __launch_bounds__(kBlock, 2) k_small_post(SmallArgs s) {
+  const StepArgs& a = s.a;
+  const int bid = blockIdx.x, G = gridDim.x;
+  unsigned want = s.base;
+  const auto barrier = [&] {
+    want += G;
+    return G == 1 ? (__syncthreads(), true) : coop::grid_barrier(s.arrived, want, &a.out->cg.err);
+  };
+  const double* const dtgp = &a.out->next_dt;
+  closure_corr_body(a.d, a.f, a.x, a.hn, a.hp, a.kcx, a.kcy, a.kcz, bid, G);
+  if (!barrier()) return;
+  const PassK pk{a.kcx, a.kcy, a.kcz, a.wcn};
+  flux_body<false, false>(a.d, a.f, pk, a.hp, a.wcn, a.kx, a.ky, a.kzf, a.qx, a.qy, a.qzf, dtgp, bid,
+                          G);
+  if (!barrier()) return;
+  update_wc_body<false>(a.d, a.f, a.hp, a.hn, a.wcn, a.qx, a.qy, a.qzf, dtgp, a.wcu, a.satf,
+                        a.colflag, a.partial + kPSs * G, bid, G);
+  if (!barrier()) return;
+  classify_body<false>(a.d, a.f, a.kx, a.ky, a.kzf, a.wcu, a.hp, a.satf, a.wc_out, a.h_out, a.room,
+                       a.sup, a.sdn, a.colflag, a.partial + kPAdj * G, a.partial + kPDrop * G, bid,
+                       G);
+  if (!barrier()) return;
+  if (a.warp_walk)
+    walk_body<false>(a.d, a.f, a.wc_out, a.room, a.sup, a.sdn, a.qzf, a.colflag, dtgp, a.partial, G,
+                     nullptr, nullptr, bid, G);
+  else
+    walk_thread_body<false>(a.d, a.f, a.wc_out, a.room, a.sup, a.sdn, a.qzf, a.colflag, dtgp,
+                            a.partial, G, nullptr, nullptr, bid, G);
+  if (!barrier()) return;
+  finalize_body(a.d, a.f, a.wc_out, a.vloss, a.qx, a.qy, a.qzf, dtgp, a.co_max, a.partial, G, bid,
+                G);
+  if (!barrier() || bid != 0) return;
+  const double dtg = *dtgp;  // read by every thread before thread 0 replaces it
+  step_info_body(a.partial, G, a.d.off, 0, a.dq_grow, a.dq_shrink, a.dt_min, a.dt_max, dtg, a.out);
+  __syncthreads();
+  const unsigned* src = reinterpret_cast<const unsigned*>(a.out);
+  unsigned* dst = reinterpret_cast<unsigned*>(s.host);
+  for (int w = threadIdx.x; w < static_cast<int>(sizeof(StepOut) / 4); w += blockDim.x)
+    dst[w] = src[w];
 }
 
 }  // namespace
@@ -2554,6 +2693,76 @@ cudaError_t batch_corrector(const PhaseTables& t, cudaStream_t s) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(t.outs_host, t.outs, sizeof(StepOut) * t.n, cudaMemcpyDeviceToHost, s);
+}
+
+// ---------------------------------------------------------------- small domains
+namespace {
+
+// Barriers a launch of each kernel passes (k_small_pre: without the factor).
+constexpr unsigned kPreBarriers = 3, kPostBarriers = 6;
+
+SmallArgs small_args(const Device& D, bool mixed, double dtg) {
+  SmallArgs s;
+  std::memset(&s, 0, sizeof(s));
+  fill_step_args(D, mixed, dtg, 0.0, 0.0, 0.0, 0.0, 0.0, s.a);
+  return s;
+}
+
+int small_grid(const Device& D) {
+  return static_cast<int>(std::max(1LL, std::min<long long>((D.d.ncell + kBlock - 1) / kBlock,
+                                                            std::min(D.nblk, 2 * D.sm_count))));
+}
+
+}  // namespace
+
+bool small_domain(const Device& D) {
+  return D.d.ncell <= kSmallCells && !D.f.cpl && !D.f.baro && !D.win_x;
+}
+
+cudaError_t launch_small_pre(Device& D, bool mixed, bool warm, double dtg, const double* hprev,
+                             double ratio) {
+  SmallArgs s = small_args(D, mixed, dtg);
+  s.warm = warm ? 1 : 0;
+  s.hprev = warm ? hprev : nullptr;
+  s.ratio = ratio;
+  const int G = small_grid(D);
+  s.arrived = D.small_sync;
+  s.base = D.small_base[0];
+  void* args[] = {&s};
+  ++D.launches;
+  const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_small_pre),
+                                                    dim3(G), dim3(kBlock), args, 0, D.stream);
+  if (e == cudaSuccess && G > 1)
+    D.small_base[0] += static_cast<unsigned>(G) * (kPreBarriers + (mixed ? 1 : 0));
+  return e;
+}
+
+cudaError_t launch_small_post(Device& D, double co_max, double dq_grow, double dq_shrink,
+                              double dt_min, double dt_max) {
+  SmallArgs s = small_args(D, false, 0.0);
+  s.a.co_max = co_max;
+  s.a.dq_grow = dq_grow;
+  s.a.dq_shrink = dq_shrink;
+  s.a.dt_min = dt_min;
+  s.a.dt_max = dt_max;
+  const int G = small_grid(D);
+  s.arrived = D.small_sync + 32;  // a line of its own
+  s.base = D.small_base[1];
+  s.host = D.out_host;
+  const size_t smem = s.a.warp_walk ? kWalkWarps * walk_warp_bytes(D.d.nz) : 0;
+  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_small_post), smem);
+  if (e != cudaSuccess) return e;
+  void* args[] = {&s};
+  ++D.launches;
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_small_post), dim3(G),
+                                  dim3(kBlock), args, smem, D.stream);
+  if (e == cudaSuccess && G > 1) D.small_base[1] += static_cast<unsigned>(G) * kPostBarriers;
+  return e;
+}
+
+cudaError_t reset_small_sync(Device& D) {
+  D.small_base[0] = D.small_base[1] = 0;
+  return cudaMemsetAsync(D.small_sync, 0, kSmallSyncWords * sizeof(unsigned), D.stream);
 }
 
 }  // namespace fgw

@@ -12,7 +12,7 @@
 // at every scan step (the map is projective), so nothing overflows.
 #pragma once
 
-#include "gw_device.cuh"
+#include "gw_internal.h"
 #include "gw_linesolve.cuh"
 
 namespace fgw {
@@ -41,8 +41,7 @@ __device__ inline M2 m2_mul(const M2& x, const M2& y) {  // x * y
 // columns in chunks of LPC E cells (LPC = 32), the recurrence and the last
 // cell carried from chunk to chunk.
 template <typename T, int LPC, int E, bool DEEP>
-__device__ __forceinline__ void line_factor_body(const Dims& d, const double* __restrict__ diag,
-                                                 const double* __restrict__ gzp,
+__device__ __forceinline__ void line_factor_body(const Dims& d, const double* diag, const double* gzp,
                                                  T* __restrict__ s_out, T* __restrict__ l_out,
                                                  const int bid, const int G) {
   constexpr int kCols = 32 / LPC;
@@ -119,6 +118,17 @@ __device__ __forceinline__ void line_factor_body(const Dims& d, const double* __
         m0 = 1.0;
       }
     }
+  }
+}
+
+// The FP32 factorization of one domain from its step record, by its depth.
+__device__ __forceinline__ void line_factor_any(const StepArgs& a, const int bid, const int G) {
+  switch (line_variant(a.d.nz)) {
+    case 0: line_factor_body<float, 8, 4, false>(a.d, a.diag, a.gzp, a.s32, a.l32, bid, G); break;
+    case 1: line_factor_body<float, 16, 4, false>(a.d, a.diag, a.gzp, a.s32, a.l32, bid, G); break;
+    case 2: line_factor_body<float, 32, 4, false>(a.d, a.diag, a.gzp, a.s32, a.l32, bid, G); break;
+    case 3: line_factor_body<float, 32, 8, false>(a.d, a.diag, a.gzp, a.s32, a.l32, bid, G); break;
+    default: line_factor_body<float, 32, 8, true>(a.d, a.diag, a.gzp, a.s32, a.l32, bid, G);
   }
 }
 

@@ -271,7 +271,8 @@ size_t frehg_gw_device_bytes(const frehg_gw_desc* d) {
   if (line64) b += 5 * r(8 * np) + r(8 * ns);
   const size_t nblk = std::min<size_t>((n3 + 255) / 256, 512 * 8);
   const size_t cg = std::max<size_t>((n3 + 255) / 256, 512 * 4);
-  b += r(8 * fgw::kPSlots * nblk) + r(8 * fgw::kSolveSlots * cg) + r(sizeof(fgw::StepOut));
+  b += r(8 * fgw::kPSlots * nblk) + r(8 * fgw::kSolveSlots * cg) + r(sizeof(fgw::StepOut)) +
+       r(sizeof(unsigned) * fgw::kSmallSyncWords);
   const size_t page = 2u << 20;
   return (b + page - 1) / page * page;
 }
