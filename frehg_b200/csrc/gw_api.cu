@@ -373,6 +373,14 @@ int frehg_gw_create(const frehg_gw_desc* desc, frehg_gw_handle** out) {
                   std::string("frehg_gw_create: ") + cudaGetErrorString(e));
     }
 
+    const auto same_ks = [&](int g) {
+      if (soil_kind[0] == fgw::kSoilUniform && soil_kind[g] == fgw::kSoilUniform)
+        return soil_u[0] == soil_u[g];
+      return (g == 1 ? D.ksy : D.ksz) == D.ksx;
+    };
+    d.iso = (same_ks(1) ? fgw::kIsoY : 0) | (same_ks(2) ? fgw::kIsoZ : 0);
+    if (d.iso & fgw::kIsoY) D.kcy = D.kcx;
+    if (d.iso & fgw::kIsoZ) D.kcz = D.kcx;
     fgw::Fields& f = D.f;
     {
       const double* sp[8] = {D.ksx, D.ksy, D.ksz, D.vga, D.vgn, D.wcs, D.wcr, D.aev};

@@ -31,10 +31,32 @@ struct Dims {
   double idx, idy;       // 1 / dx, 1 / dy
   double ss;             // specific storage
   int full3d, pc, harm, off, redistribute, terrain;
+  int iso;               // kIsoY / kIsoZ: Ksy / Ksz equal Ksx everywhere
   // Multipliers of the divisions by nz and by nx + 2 (div_magic); the
   // domain's cell count is below 2^32.
   unsigned long long mz, mx2;
 };
+
+// With equal conductivities the per-cell K(h, Ks) of the directions are one
+// field: it is evaluated, stored and read once (the kcy / kcz of a pass are
+// its kcx).
+enum : int { kIsoY = 1, kIsoZ = 2 };
+
+// The default scheme (consistent form, arithmetic faces, full 3D), fixed at
+// compile time: the face kernels then load neither Ks nor theta.
+template <bool PLAIN>
+__device__ inline Dims scheme(const Dims& d) {
+  Dims p = d;
+  if (PLAIN) {
+    p.pc = 1;
+    p.harm = 0;
+    p.full3d = 1;
+  }
+  return p;
+}
+__host__ __device__ inline bool plain_scheme(const Dims& d) {
+  return d.pc && !d.harm && d.full3d;
+}
 
 // The coupled top's device state (GwCoupling), one per coupled domain: the
 // vent rule, min_depth, the mesh bed (offset frame) and the surface fields

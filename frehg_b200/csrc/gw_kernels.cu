@@ -189,12 +189,12 @@ __device__ __forceinline__ void closure_pred_body(Dims d, Fields f,
        c += static_cast<long long>(G) * blockDim.x) {
     const double hc = h[c];
     const Soil so = soil_at(f, c);
-    const double ksx = f.ksx[c], ksy = f.ksy[c], ksz = f.ksz[c];
+    const double ksx = f.ksx[c];
     const VgParts v = vg_parts(so, hc);
     const KrParts p = vg_kr_from(v, hc);
     kcx[c] = vg_k_from(p, ksx);
-    kcy[c] = vg_k_from(p, ksy);
-    kcz[c] = vg_k_from(p, ksz);
+    if (!(d.iso & kIsoY)) kcy[c] = vg_k_from(p, f.ksy[c]);
+    if (!(d.iso & kIsoZ)) kcz[c] = vg_k_from(p, f.ksz[c]);
     ch[c] = vg_capacity_from(so, v, hc);
   }
 }
@@ -261,13 +261,13 @@ __device__ __forceinline__ void closure_corr_body(Dims d, Fields f,
     int j, i, k;
     unflatten(d, c, j, i, k);
     const Soil so = soil_at(f, c);
-    const double ksx = f.ksx[c], ksy = f.ksy[c], ksz = f.ksz[c];
+    const double ksx = f.ksx[c];
     const double hv = predicted_head(d, f, x, hn, c, j, i);
     const KrParts p = vg_kr_parts(so, hv);
     hp[c] = hv;
     kcx[c] = vg_k_from(p, ksx);
-    kcy[c] = vg_k_from(p, ksy);
-    kcz[c] = vg_k_from(p, ksz);
+    if (!(d.iso & kIsoY)) kcy[c] = vg_k_from(p, f.ksy[c]);
+    if (!(d.iso & kIsoZ)) kcz[c] = vg_k_from(p, f.ksz[c]);
   }
 }
 
@@ -590,10 +590,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_assemble(
 // j = 0) and the z face above it (plus the bottom face for k = nz-1), into
 // the face arrays the corrector's k_flux overwrites later in the step.  A
 // separate pass keeps the assembly's loads to six face values.
-template <bool CPL>
-__device__ __forceinline__ void faces_body(Dims d, Fields f, PassK pk, double* __restrict__ kx,
+template <bool CPL, bool PLAIN>
+__device__ __forceinline__ void faces_body(Dims dd, Fields f, PassK pk, double* __restrict__ kx,
                                            double* __restrict__ ky, double* __restrict__ kzf,
                                            const int bid, const int G) {
+  const Dims d = scheme<PLAIN>(dd);
   for (long long c = bid * static_cast<long long>(blockDim.x) + threadIdx.x; c < d.ncell;
        c += static_cast<long long>(G) * blockDim.x) {
     int j, i, k;
@@ -617,7 +618,7 @@ __device__ __forceinline__ void faces_body(Dims d, Fields f, PassK pk, double* _
       const long long col = col2(d, j, i), fz = fidx(d, j, i, k);
       const long long cu = (k >= 1) ? c - 1 : c;
       const ZFlank zu{pk.kcz[cu], f.ksz[cu], f.dz[cu], (k >= 1) ? f.act[cu] : int8_t(0)};
-      const ZFlank zc{pk.kcz[c], f.ksz[c], f.dz[c], f.act[c]};
+      const ZFlank zc{pk.kcz[c], (PLAIN && k > 0) ? 0.0 : f.ksz[c], f.dz[c], f.act[c]};
       const int topc = f.topc[col], botc = f.botc[col];
       const double dep = (CPL && k == 0) ? f.cpl->dept[col] : 0.0;
       kzf[fz] = face_z<CPL>(d, zu, zc, k, topc, botc, dep);
@@ -629,10 +630,10 @@ __device__ __forceinline__ void faces_body(Dims d, Fields f, PassK pk, double* _
   }
 }
 
-template <bool CPL>
+template <bool CPL, bool PLAIN>
 __global__ void __launch_bounds__(kBlock, 4) k_faces(Dims d, Fields f, PassK pk, double* kx,
                                                      double* ky, double* kzf) {
-  faces_body<CPL>(d, f, pk, kx, ky, kzf, blockIdx.x, gridDim.x);
+  faces_body<CPL, PLAIN>(d, f, pk, kx, ky, kzf, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------- fluxes
@@ -777,8 +778,8 @@ __device__ inline double flux_top_coupled(const Dims& d, const Fields& f, long l
 // boundary faces through the ghost cells i = 0, j = 0) and the z face above
 // it (plus the bottom face for k = nz-1).  Each face's loads are issued
 // before its rules run.
-template <bool CPL, bool BARO>
-__device__ __forceinline__ void flux_body(Dims d, Fields f, PassK pk,
+template <bool CPL, bool BARO, bool PLAIN>
+__device__ __forceinline__ void flux_body(Dims dd, Fields f, PassK pk,
                                                     const double* __restrict__ hp,
                                                     const double* __restrict__ wcn,
                                                     double* __restrict__ kx,
@@ -789,6 +790,7 @@ __device__ __forceinline__ void flux_body(Dims d, Fields f, PassK pk,
                                                     double* __restrict__ qzf,
                                                     const double* __restrict__ dtgp,
                                                     const int bid, const int G) {
+  const Dims d = scheme<PLAIN>(dd);
   const double dtg = CPL ? *dtgp : 0.0;
   for (long long c = bid * static_cast<long long>(blockDim.x) + threadIdx.x; c < d.ncell;
        c += static_cast<long long>(G) * blockDim.x) {
@@ -823,7 +825,10 @@ __device__ __forceinline__ void flux_body(Dims d, Fields f, PassK pk,
     if (doZ) {
       const long long col = col2(d, j, i);
       zu = ZFlank{pk.kcz[cu], f.ksz[cu], f.dz[cu], (k >= 1) ? f.act[cu] : int8_t(0)};
-      zc = ZFlank{pk.kcz[c], f.ksz[c], f.dz[c], f.act[c]};
+      // Ks is read for the face above a column's top cell only: on the terrain
+      // mesh, whose columns are whole, the cells k = 0.
+      const bool ks = !PLAIN || CPL || k == 0 || !d.terrain;
+      zc = ZFlank{pk.kcz[c], ks ? f.ksz[c] : 0.0, f.dz[c], f.act[c]};
       hpu = hp[cu];
       hpc = hp[c];
       topc = f.topc[col];
@@ -865,7 +870,7 @@ __device__ __forceinline__ void flux_body(Dims d, Fields f, PassK pk,
   }
 }
 
-template <bool CPL, bool BARO>
+template <bool CPL, bool BARO, bool PLAIN>
 __global__ void __launch_bounds__(kBlock, 2) k_flux(Dims d, Fields f, PassK pk,
                                                     const double* __restrict__ hp,
                                                     const double* __restrict__ wcn,
@@ -876,7 +881,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_flux(Dims d, Fields f, PassK pk,
                                                     double* __restrict__ qy,
                                                     double* __restrict__ qzf,
                                                     const double* __restrict__ dtgp) {
-  flux_body<CPL, BARO>(d, f, pk, hp, wcn, kx, ky, kzf, qx, qy, qzf, dtgp, blockIdx.x, gridDim.x);
+  flux_body<CPL, BARO, PLAIN>(d, f, pk, hp, wcn, kx, ky, kzf, qx, qy, qzf, dtgp, blockIdx.x, gridDim.x);
 }
 
 // ---------------------------------------------------------------- theta update
@@ -1150,9 +1155,14 @@ __device__ __forceinline__ void classify_body(
     }
     wc_out[c] = r.wout;
     h_out[c] = r.hout;
-    room[c] = r.rm;
-    sup[c] = r.up;
-    sdn[c] = r.dn;
+    // The warp walk (room null) takes the room from theta again and reads the
+    // surplus of saturated cells only, where it can be (or, redistributing,
+    // of all): three words a cell less for most of a domain.
+    if (room) room[c] = r.rm;
+    if (room || d.redistribute || r.wout >= f.wcs[c]) {
+      sup[c] = r.up;
+      sdn[c] = r.dn;
+    }
   }
   const RedItem it[2] = {{adj, kRedSum, part_adj + bid}, {drop, kRedSum, part_drop + bid}};
   block_reduce_many(it);
@@ -1480,8 +1490,7 @@ __device__ inline void walk_cell(const Dims& d, int kk, double upv, double dnv, 
 // into shared memory and the room bits; with `all` also the reciprocal cell
 // volumes and the inactive bits (a restage keeps those).
 __device__ inline void walk_stage(const Dims& d, const Fields& f, long long base, long long fb,
-                                  int nz, int lane, const double* __restrict__ room,
-                                  const double* wc, const double* qzf, double* rs, double* ws,
+                                  int nz, int lane, const double* wc, const double* qzf, double* rs, double* ws,
                                   double* ivs, double* qs, unsigned* rbits, unsigned* ibits,
                                   bool all) {
   for (int k0 = 0; k0 < nz; k0 += 32) {
@@ -1489,9 +1498,11 @@ __device__ inline void walk_stage(const Dims& d, const Fields& f, long long base
     double r = 0.0;
     bool inact = false;
     if (k < nz) {
-      r = room[base + k];
+      const double w = wc[base + k];
+      // the classification's room of the cell
+      r = f.act[base + k] ? (f.wcs[base + k] - w) * (d.az * f.dz[base + k]) : 0.0;
       rs[k] = r;
-      ws[k] = wc[base + k];
+      ws[k] = w;
       if (all) ivs[k] = 1.0 / (d.az * f.dz[base + k]);
       inact = !f.act[base + k];
     }
@@ -1521,15 +1532,16 @@ __device__ inline void walk_stage(const Dims& d, const Fields& f, long long base
 // restored, the caller restages the column and runs the general walk.
 __device__ inline int walk_fast(const Fields& f, long long base, int nz, int lane, double* rs,
                                 double* ws, const double* ivs, double* qs, const unsigned* rbits,
-                                const unsigned* ibits, const double* __restrict__ sup,
-                                const double* __restrict__ sdn, double idtg, double& lost) {
+                                const unsigned* ibits, const double* wc, bool redistribute,
+                                const double* __restrict__ sup, const double* __restrict__ sdn,
+                                double idtg, double& lost) {
   const double lost0 = lost;
   for (int k0 = 0; k0 < nz; k0 += 32) {
     const int k = k0 + lane;
     double su = 0.0, sd = 0.0;
     int mu = -1, md = -1;
     bool any = false, bad = false;
-    if (k < nz && f.act[base + k]) {
+    if (k < nz && f.act[base + k] && (redistribute || wc[base + k] >= f.wcs[base + k])) {
       su = sup[base + k];
       sd = sdn[base + k];
       any = su > 0.0 || sd > 0.0;
@@ -1588,7 +1600,6 @@ __device__ inline int walk_fast(const Fields& f, long long base, int nz, int lan
 
 template <bool CPL>
 __device__ __forceinline__ void walk_body(Dims d, Fields f, double* wc,
-                                                 const double* __restrict__ room,
                                                  const double* __restrict__ sup,
                                                  const double* __restrict__ sdn, double* qzf,
                                                  const int* __restrict__ colflag,
@@ -1620,23 +1631,25 @@ __device__ __forceinline__ void walk_body(Dims d, Fields f, double* wc,
     double* pc = pcorr ? pcorr + fb : nullptr;  // transport window: this column's path records
     if (pc)
       for (int q = lane; q <= nz; q += 32) pc[q] = 0.0;
-    walk_stage(d, f, base, fb, nz, lane, room, wc, qzf, rs, ws, ivs, qs, rbits, ibits, true);
+    walk_stage(d, f, base, fb, nz, lane, wc, qzf, rs, ws, ivs, qs, rbits, ibits, true);
     int how = 1;
     if (!CPL && !pc)
-      how = walk_fast(f, base, nz, lane, rs, ws, ivs, qs, rbits, ibits, sup, sdn, idtg, lost);
+      how = walk_fast(f, base, nz, lane, rs, ws, ivs, qs, rbits, ibits, wc, d.redistribute,
+                      sup, sdn, idtg, lost);
     if (how == 0) {
       for (int k = lane; k < nz; k += 32) wc[base + k] = ws[k];
       for (int k = lane; k <= nz; k += 32) qzf[fb + k] = qs[k];
       __syncwarp();
       continue;
     }
-    if (how == 2) walk_stage(d, f, base, fb, nz, lane, room, wc, qzf, rs, ws, ivs, qs, rbits, ibits,
+    if (how == 2) walk_stage(d, f, base, fb, nz, lane, wc, qzf, rs, ws, ivs, qs, rbits, ibits,
                              false);
     for (int k0 = 0; k0 < nz; k0 += 32) {
       const int k = k0 + lane;
       double su = 0.0, sd = 0.0;
       bool any = false;
-      if (k < nz && f.act[base + k]) {
+      // wc still holds the classification's theta (the walk's is in ws)
+      if (k < nz && f.act[base + k] && (d.redistribute || wc[base + k] >= f.wcs[base + k])) {
         su = sup[base + k];
         sd = sdn[base + k];
         any = su > 0.0 || sd > 0.0;
@@ -1668,14 +1681,13 @@ __device__ __forceinline__ void walk_body(Dims d, Fields f, double* wc,
 // minimum ptxas settled on 64 / 80 registers with spills.
 template <bool CPL>
 __global__ void __launch_bounds__(kBlock, CPL ? 3 : 4) k_walk(Dims d, Fields f, double* wc,
-                                                 const double* __restrict__ room,
                                                  const double* __restrict__ sup,
                                                  const double* __restrict__ sdn, double* qzf,
                                                  const int* __restrict__ colflag,
                                                  const double* __restrict__ dtgp,
                                                  double* partial, int nblk, double* pcorr,
                                                  double* wvent) {
-  walk_body<CPL>(d, f, wc, room, sup, sdn, qzf, colflag, dtgp, partial, nblk, pcorr, wvent,
+  walk_body<CPL>(d, f, wc, sup, sdn, qzf, colflag, dtgp, partial, nblk, pcorr, wvent,
                  blockIdx.x, gridDim.x);
 }
 
@@ -2168,7 +2180,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_faces_batch(const StepArgs* tab, 
   int bid, G;
   load_member(tab, first, n, sa, bid, G);
   const PassK pk{sa.kcx, sa.kcy, sa.kcz, sa.wcn};
-  faces_body<false>(sa.d, sa.f, pk, sa.kx, sa.ky, sa.kzf, bid, G);
+  if (plain_scheme(sa.d)) faces_body<false, true>(sa.d, sa.f, pk, sa.kx, sa.ky, sa.kzf, bid, G);
+  else faces_body<false, false>(sa.d, sa.f, pk, sa.kx, sa.ky, sa.kzf, bid, G);
 }
 
 __global__ void __launch_bounds__(kBlock) k_closure_corr_batch(const StepArgs* tab,
@@ -2185,8 +2198,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_flux_batch(const StepArgs* tab, c
   int bid, G;
   load_member(tab, first, n, sa, bid, G);
   const PassK pk{sa.kcx, sa.kcy, sa.kcz, sa.wcn};
-  flux_body<false, false>(sa.d, sa.f, pk, sa.hp, sa.wcn, sa.kx, sa.ky, sa.kzf, sa.qx, sa.qy, sa.qzf, &sa.dtg, bid,
-            G);
+  if (plain_scheme(sa.d))
+    flux_body<false, false, true>(sa.d, sa.f, pk, sa.hp, sa.wcn, sa.kx, sa.ky, sa.kzf, sa.qx, sa.qy,
+                                  sa.qzf, &sa.dtg, bid, G);
+  else
+    flux_body<false, false, false>(sa.d, sa.f, pk, sa.hp, sa.wcn, sa.kx, sa.ky, sa.kzf, sa.qx,
+                                   sa.qy, sa.qzf, &sa.dtg, bid, G);
 }
 
 __global__ void __launch_bounds__(kBlock, 4) k_update_wc_batch(const StepArgs* tab,
@@ -2204,7 +2221,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_classify_batch(const StepArgs* ta
   int bid, G;
   load_member(tab, first, n, sa, bid, G);
   classify_body<false>(sa.d, sa.f, sa.kx, sa.ky, sa.kzf, sa.wcu, sa.hp, sa.satf, sa.wc_out, sa.h_out,
-                sa.room, sa.sup, sa.sdn, sa.colflag, sa.partial + kPAdj * sa.nblk,
+                sa.warp_walk ? nullptr : sa.room, sa.sup, sa.sdn, sa.colflag, sa.partial + kPAdj * sa.nblk,
                 sa.partial + kPDrop * sa.nblk, bid, G);
 }
 
@@ -2214,7 +2231,7 @@ __global__ void __launch_bounds__(kBlock) k_walk_batch(const StepArgs* tab, cons
   int bid, G;
   load_member(tab, first, n, sa, bid, G);
   if (sa.warp_walk) {
-    walk_body<false>(sa.d, sa.f, sa.wc_out, sa.room, sa.sup, sa.sdn, sa.qzf, sa.colflag, &sa.dtg,
+    walk_body<false>(sa.d, sa.f, sa.wc_out, sa.sup, sa.sdn, sa.qzf, sa.colflag, &sa.dtg,
               sa.partial, sa.nblk, nullptr, nullptr, bid, G);
   } else {
     walk_thread_body<false>(sa.d, sa.f, sa.wc_out, sa.room, sa.sup, sa.sdn, sa.qzf, sa.colflag, &sa.dtg,
@@ -2290,7 +2307,8 @@ __global__ void __launch_bounds__(kBlock, 2) k_small_pre(SmallArgs s) {
   closure_pred_body(a.d, a.f, a.hn, a.kcx, a.kcy, a.kcz, a.ch, bid, G);
   if (!barrier()) return;
   const PassK pk{a.kcx, a.kcy, a.kcz, a.wcn};
-  faces_body<false>(a.d, a.f, pk, a.kx, a.ky, a.kzf, bid, G);
+  if (plain_scheme(a.d)) faces_body<false, true>(a.d, a.f, pk, a.kx, a.ky, a.kzf, bid, G);
+  else faces_body<false, false>(a.d, a.f, pk, a.kx, a.ky, a.kzf, bid, G);
   if (!barrier()) return;
   assemble_body<false, false>(a.d, a.f, a.kx, a.ky, a.kzf, a.hn, a.wcn, a.ch, &a.out->next_dt,
                               a.diag, a.gxp, a.gyp, a.gzp, a.rhs, s.warm ? a.x : nullptr, s.hprev,
@@ -2312,18 +2330,22 @@ __global__ void __launch_bounds__(kBlock, 2) k_small_post(SmallArgs s) {
   closure_corr_body(a.d, a.f, a.x, a.hn, a.hp, a.kcx, a.kcy, a.kcz, bid, G);
   if (!barrier()) return;
   const PassK pk{a.kcx, a.kcy, a.kcz, a.wcn};
-  flux_body<false, false>(a.d, a.f, pk, a.hp, a.wcn, a.kx, a.ky, a.kzf, a.qx, a.qy, a.qzf, dtgp, bid,
-                          G);
+  if (plain_scheme(a.d))
+    flux_body<false, false, true>(a.d, a.f, pk, a.hp, a.wcn, a.kx, a.ky, a.kzf, a.qx, a.qy, a.qzf,
+                                  dtgp, bid, G);
+  else
+    flux_body<false, false, false>(a.d, a.f, pk, a.hp, a.wcn, a.kx, a.ky, a.kzf, a.qx, a.qy, a.qzf,
+                                   dtgp, bid, G);
   if (!barrier()) return;
   update_wc_body<false>(a.d, a.f, a.hp, a.hn, a.wcn, a.qx, a.qy, a.qzf, dtgp, a.wcu, a.satf,
                         a.colflag, a.partial + kPSs * G, bid, G);
   if (!barrier()) return;
-  classify_body<false>(a.d, a.f, a.kx, a.ky, a.kzf, a.wcu, a.hp, a.satf, a.wc_out, a.h_out, a.room,
-                       a.sup, a.sdn, a.colflag, a.partial + kPAdj * G, a.partial + kPDrop * G, bid,
+  classify_body<false>(a.d, a.f, a.kx, a.ky, a.kzf, a.wcu, a.hp, a.satf, a.wc_out, a.h_out,
+                       a.warp_walk ? nullptr : a.room, a.sup, a.sdn, a.colflag, a.partial + kPAdj * G, a.partial + kPDrop * G, bid,
                        G);
   if (!barrier()) return;
   if (a.warp_walk)
-    walk_body<false>(a.d, a.f, a.wc_out, a.room, a.sup, a.sdn, a.qzf, a.colflag, dtgp, a.partial, G,
+    walk_body<false>(a.d, a.f, a.wc_out, a.sup, a.sdn, a.qzf, a.colflag, dtgp, a.partial, G,
                      nullptr, nullptr, bid, G);
   else
     walk_thread_body<false>(a.d, a.f, a.wc_out, a.room, a.sup, a.sdn, a.qzf, a.colflag, dtgp,
@@ -2393,8 +2415,9 @@ void launch_closure_pred(const Device& D, const double* h) {
 void launch_assemble(const Device& D, const double* hn, const double* wcn, bool warm,
                      const double* hprev, double ratio) {
   const PassK pk{D.kcx, D.kcy, D.kcz, wcn};
-  const auto faces = (D.f.cpl != nullptr) ? k_faces<true> : k_faces<false>;
-  const bool cpl = D.f.cpl != nullptr, baro = D.f.baro != nullptr;
+  const bool cpl = D.f.cpl != nullptr, baro = D.f.baro != nullptr, plain = plain_scheme(D.d);
+  const auto faces = cpl ? (plain ? k_faces<true, true> : k_faces<true, false>)
+                         : (plain ? k_faces<false, true> : k_faces<false, false>);
   const auto assemble = cpl ? (baro ? k_assemble<true, true> : k_assemble<true, false>)
                             : (baro ? k_assemble<false, true> : k_assemble<false, false>);
   faces<<<cells_grid(D), kBlock, 0, D.stream>>>(D.d, D.f, pk, D.kx, D.ky, D.kzf);
@@ -2414,8 +2437,12 @@ void launch_closure_corr(const Device& D, const double* hn) {
 void launch_flux(const Device& D, const double* wcn) {
   PassK pk{D.kcx, D.kcy, D.kcz, wcn};
   const bool cpl = D.f.cpl != nullptr, baro = D.f.baro != nullptr;
-  const auto flux = cpl ? (baro ? k_flux<true, true> : k_flux<true, false>)
-                        : (baro ? k_flux<false, true> : k_flux<false, false>);
+  const bool plain = plain_scheme(D.d);
+  const auto flux = cpl ? (baro ? (plain ? k_flux<true, true, true> : k_flux<true, true, false>)
+                                : (plain ? k_flux<true, false, true> : k_flux<true, false, false>))
+                        : (baro ? (plain ? k_flux<false, true, true> : k_flux<false, true, false>)
+                                : (plain ? k_flux<false, false, true>
+                                         : k_flux<false, false, false>));
   flux<<<cells_grid(D), kBlock, 0, D.stream>>>(D.d, D.f, pk, D.hp, wcn, D.kx, D.ky, D.kzf, D.qx,
                                                  D.qy, D.qzf, dtg_slot(D));
   ++D.launches;
@@ -2429,27 +2456,34 @@ void launch_update_wc(const Device& D, const double* hn, const double* wcn) {
   ++D.launches;
 }
 
-void launch_classify(const Device& D, double* wc_out, double* h_out) {
-  const auto classify = (D.f.baro != nullptr) ? k_classify<true> : k_classify<false>;
-  classify<<<cells_grid(D), kBlock, 0, D.stream>>>(
-      D.d, D.f, D.kx, D.ky, D.kzf, D.wcu, D.hp, D.satf, wc_out, h_out, D.room, D.sup, D.sdn,
-      D.colflag,
-      D.partial + kPAdj * D.nblk, D.partial + kPDrop * D.nblk);
-  ++D.launches;
-}
-
 // Columns up to kWalkMaxNz cells take the warp walk (dynamic shared memory
 // opted in up to kWalkSmemMax); deeper columns take the per-thread walk.
 constexpr int kWalkMaxNz = 256;
 constexpr size_t kWalkSmemMax = 96 * 1024;
 
+bool warp_walk(const Device& D) {
+  return D.d.nz <= kWalkMaxNz && kWalkWarps * walk_warp_bytes(D.d.nz) <= kWalkSmemMax;
+}
+
+void launch_classify(const Device& D, double* wc_out, double* h_out) {
+  const auto classify = (D.f.baro != nullptr) ? k_classify<true> : k_classify<false>;
+  classify<<<cells_grid(D), kBlock, 0, D.stream>>>(
+      D.d, D.f, D.kx, D.ky, D.kzf, D.wcu, D.hp, D.satf, wc_out, h_out,
+      warp_walk(D) ? nullptr : D.room, D.sup, D.sdn,
+      D.colflag,
+      D.partial + kPAdj * D.nblk, D.partial + kPDrop * D.nblk);
+  ++D.launches;
+}
+
 void launch_walk(const Device& D, double* wc_out) {
   const size_t smem = kWalkWarps * walk_warp_bytes(D.d.nz);
-  if (D.d.nz <= kWalkMaxNz && smem <= kWalkSmemMax &&
-      raise_smem_limit(reinterpret_cast<const void*>((D.f.cpl != nullptr) ? k_walk<true> : k_walk<false>),
-                       smem) == cudaSuccess) {
+  if (warp_walk(D)) {
+    // (the classification has left out what the thread walk would need; the
+    // limit, at most kWalkSmemMax, holds on every B200)
+    raise_smem_limit(reinterpret_cast<const void*>((D.f.cpl != nullptr) ? k_walk<true> : k_walk<false>),
+                     smem);
     const auto walk = (D.f.cpl != nullptr) ? k_walk<true> : k_walk<false>;
-    walk<<<cells_grid(D), kBlock, smem, D.stream>>>(D.d, D.f, wc_out, D.room, D.sup, D.sdn,
+    walk<<<cells_grid(D), kBlock, smem, D.stream>>>(D.d, D.f, wc_out, D.sup, D.sdn,
                                                       D.qzf, D.colflag, dtg_slot(D), D.partial,
                                                       D.nblk, D.pcorr, D.win_vent);
   } else {
@@ -2609,8 +2643,7 @@ void fill_step_args(const Device& D, bool mixed, double dtg, double co_max, doub
   a.dt_max = dt_max;
   a.nblk = batch_cell_blocks(D);
   a.mixed = mixed ? 1 : 0;
-  const size_t smem = kWalkWarps * walk_warp_bytes(D.d.nz);
-  a.warp_walk = (D.d.nz <= kWalkMaxNz && smem <= kWalkSmemMax) ? 1 : 0;
+  a.warp_walk = warp_walk(D) ? 1 : 0;
 }
 
 cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>& ds,
