@@ -29,6 +29,9 @@
 // Neighbour reads are served by L1/L2 because the grid-stride sweep keeps all
 // resident blocks inside a few j-rows of each other.
 //
+// Small domains at the usual tolerances run the one-barrier form of the same
+// iteration (cg64_one_body).
+//
 // A thread's cells stay its own for the whole solve, so the words only it
 // reads can stay in shared memory (cg64_words: as many of w, y, s and the legs
 // as the domain's size leaves room for).  512x512x128 (no room) 692 -> 571 us an
@@ -56,6 +59,7 @@ struct Cg64Args {
   const double *diag, *b;
   double *gxp, *gyp, *gzp;       // scaled in place
   double *x, *r, *z, *p0, *p1, *w;  // x holds y and z holds s until the end
+  double* bw;                       // b's array, free once r is made
   double* part;  // kRedSlots x G, zero before the launch
   CgState* st;
   double rtol, atol;
@@ -367,12 +371,284 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   }
 }
 
+// ---------------------------------------------------------------- one barrier an iteration
+// The same CG with one reduction an iteration (Chronopoulos and Gear, "s-step
+// iterative methods for symmetric linear systems", J. Comput. Appl. Math. 25,
+// 1989): with w = A r beside r, g = r'r and d = r'w,
+//   b = g / g_old,  a = g / (d - b g / a_old)        (p'Ap = d - b g / a_old)
+//   p = r + b p,  s = w + b s (= A p),  y += a p,  r -= a s,  w = A r,
+// so one pass and one barrier do what the stencil and the update pass do.  A
+// neighbour's new r is taken from its old r, w and s (three vectors read where
+// p needs two, all three in two buffers), which costs a large domain more
+// traffic than the barrier costs it; p and y must fit in shared memory beside
+// their thread.  The recurrence for s loses a little attainable accuracy, so
+// tight solves keep the two-barrier form (kOneBarrierRtol).
+// Per iteration, against the two-barrier form: 64x64x128 10.9 -> 9.8 us; a
+// 101x55x25 coupled pass 20.4 -> 16.3 ms.
+enum OneWord { kOneY = 0, kOneP, kOneS, kOneGym, kOneGxm, kOneGx, kOneGy };
+
+template <bool ALIGNED, int W, bool START, bool FIRST>
+__device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, const int words,
+                                              double al, double be, const double* ro,
+                                              const double* wo, const double* so, double* rn,
+                                              double* wn, double* sn, long long t0,
+                                              long long stride, double& rr, double& rw,
+                                              double& zz) {
+  const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy;
+  int o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
+    const long long c = 2 * q;
+    const auto chip = [&](int word) -> double2& { return own[word * words + o]; };
+    const auto leg = [&](int word, const double* g) {
+      if (W > word && !START) return chip(word);
+      const double2 v = ldp<ALIGNED>(g);
+      if (W > word) chip(word) = v;
+      return v;
+    };
+    // r - al (w + be s) of a pair (START: r; FIRST: r - al w)
+    const auto next2 = [&](long long m) {
+      double2 r = ldp<ALIGNED>(ro + m);
+      if (START) return r;
+      const double2 w = ldp<ALIGNED>(wo + m);
+      if (FIRST) {
+        r.x -= al * w.x;
+        r.y -= al * w.y;
+      } else {
+        const double2 s = ldp<ALIGNED>(so + m);
+        r.x -= al * (w.x + be * s.x);
+        r.y -= al * (w.y + be * s.y);
+      }
+      return r;
+    };
+    const auto next1 = [&](long long m) {
+      return START ? ro[m] : FIRST ? ro[m] - al * wo[m] : ro[m] - al * (wo[m] + be * so[m]);
+    };
+    const double2 rym = next2(c - sy), rxm = next2(c - sx);
+    const double2 rxp = next2(c + sx), ryp = next2(c + sy);
+    const double rkm = next1(c - 1), rkp = next1(c + 2);
+    const double2 gx = leg(kOneGx, a.gxp + c), gxm = leg(kOneGxm, a.gxp + c - sx);
+    const double2 gy = leg(kOneGy, a.gyp + c), gym = leg(kOneGym, a.gyp + c - sy);
+    const double2 gz = ldp<ALIGNED>(a.gzp + c);
+    const double gzm = a.gzp[c - 1];
+    double2 r = ldp<ALIGNED>(ro + c);
+    if (!START) {
+      double2 s = ldp<ALIGNED>(wo + c), p = r;
+      double2 y = make_double2(0.0, 0.0);
+      if (!FIRST) {
+        const double2 sp = ldp<ALIGNED>(so + c), pp = chip(kOneP);
+        y = chip(kOneY);
+        s.x += be * sp.x;
+        s.y += be * sp.y;
+        p.x += be * pp.x;
+        p.y += be * pp.y;
+      }
+      y.x += al * p.x;
+      y.y += al * p.y;
+      chip(kOneP) = p;
+      chip(kOneY) = y;
+      r.x -= al * s.x;
+      r.y -= al * s.y;
+      stp<ALIGNED>(rn + c, r.x, r.y);
+      stp<ALIGNED>(sn + c, s.x, s.y);
+      const double2 S = W > kOneS ? chip(kOneS) : ldp<ALIGNED>(a.z + c);
+      const double z0 = S.x * r.x, z1 = S.y * r.y;
+      rr += r.x * r.x;
+      rr += r.y * r.y;
+      zz += z0 * z0;
+      zz += z1 * z1;
+    }
+    double w0 = gym.x * rym.x;
+    w0 += gxm.x * rxm.x;
+    w0 += gzm * rkm;
+    w0 += r.x;
+    w0 += gz.x * r.y;
+    w0 += gx.x * rxp.x;
+    w0 += gy.x * ryp.x;
+    double w1 = gym.y * rym.y;
+    w1 += gxm.y * rxm.y;
+    w1 += gz.x * r.x;
+    w1 += r.y;
+    w1 += gz.y * rkp;
+    w1 += gx.y * rxp.y;
+    w1 += gy.y * ryp.y;
+    stp<ALIGNED>(wn + c, w0, w1);
+    rw += r.x * w0;
+    rw += r.y * w1;
+  }
+}
+
+template <bool ALIGNED, int W>
+__device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, const int G,
+                                              double2* own, const int words) {
+  static_assert(W >= 2, "y and p stay with their thread");
+  const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy, ct = a.d.ncell - 1;
+  // The last cell of an odd count, taken by the grid's last thread, with its
+  // own y, p and s in registers.
+  const bool tail = !ALIGNED && (a.d.ncell & 1) && bid == G - 1 && threadIdx.x == blockDim.x - 1;
+  const long long stride = static_cast<long long>(G) * blockDim.x;
+  const long long t0 = bid * static_cast<long long>(blockDim.x) + threadIdx.x;
+  double* const rb[2] = {a.r, a.p0};
+  double* const wb[2] = {a.w, a.p1};
+  double* const sb[2] = {a.bw, a.x};
+  unsigned epoch = 0;
+
+  double rr = 0.0, zz = 0.0, rw = 0.0, ty = 0.0, tp = 0.0, ts = 0.0;
+  int o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
+    const long long c = 2 * q;
+    const double2 bv = ldp<ALIGNED>(a.b + c), dg = ldp<ALIGNED>(a.diag + c);
+    const double2 dx = ldp<ALIGNED>(a.diag + c + sx), dy = ldp<ALIGNED>(a.diag + c + sy);
+    const double dz = a.diag[c + 2];
+    const double2 gx = ldp<ALIGNED>(a.gxp + c), gy = ldp<ALIGNED>(a.gyp + c);
+    const double2 gz = ldp<ALIGNED>(a.gzp + c);
+    const double s0 = 1.0 / sqrt(dg.x), s1 = 1.0 / sqrt(dg.y);
+    const double r0 = s0 * bv.x, r1 = s1 * bv.y;
+    stp<ALIGNED>(a.gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
+    stp<ALIGNED>(a.gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
+    stp<ALIGNED>(a.gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
+    stp<ALIGNED>(a.r + c, r0, r1);
+    if (W > kOneS) own[kOneS * words + o] = make_double2(s0, s1);
+    else stp<ALIGNED>(a.z + c, s0, s1);
+    const double z0 = s0 * r0, z1 = s1 * r1;
+    rr += r0 * r0;
+    rr += r1 * r1;
+    zz += z0 * z0;
+    zz += z1 * z1;
+    own[kOneY * words + o] = make_double2(0.0, 0.0);
+  }
+  if (tail) {
+    ts = 1.0 / sqrt(a.diag[ct]);
+    const double r = ts * a.b[ct];
+    a.r[ct] = r;
+    a.gxp[ct] *= ts / sqrt(a.diag[ct + sx]);
+    a.gyp[ct] *= ts / sqrt(a.diag[ct + sy]);
+    a.gzp[ct] *= ts / sqrt(a.diag[ct + 1]);
+    rr += r * r;
+    zz += (ts * r) * (ts * r);
+  }
+  double v2[2] = {zz, rr};
+  if (!grid_sum<kCgBlock>(v2, a.part, bid, G, epoch, a.st)) return;
+  double dp = sqrt(v2[0]), gamma = v2[1];
+  const double rnorm0 = dp;
+  const double ttol = fmax(a.rtol * rnorm0, a.atol);
+  int reason = 0, its = 0;
+  const auto test = [&](double rn) {
+    if (!isfinite(rn)) reason = -9;
+    else if (rn <= ttol) reason = (rn < a.atol) ? 3 : 2;
+    else if (rn >= 1.0e5 * rnorm0) reason = -4;
+  };
+  test(dp);
+  // The tail cell's share of a pass, on the buffers the pairs use.
+  const auto tail_cell = [&](bool start, bool first, double al, double be, const double* ro,
+                             const double* wo, const double* so, double* rn, double* wn,
+                             double* sn) {
+    const auto nx = [&](long long m) {
+      return start ? ro[m] : first ? ro[m] - al * wo[m] : ro[m] - al * (wo[m] + be * so[m]);
+    };
+    double r = ro[ct];
+    if (!start) {
+      const double s = first ? wo[ct] : wo[ct] + be * so[ct];
+      tp = first ? r : r + be * tp;
+      ty += al * tp;
+      r -= al * s;
+      rn[ct] = r;
+      sn[ct] = s;
+      rr += r * r;
+      zz += (ts * r) * (ts * r);
+    }
+    double wv = a.gyp[ct - sy] * nx(ct - sy);
+    wv += a.gxp[ct - sx] * nx(ct - sx);
+    wv += a.gzp[ct - 1] * nx(ct - 1);
+    wv += r;
+    wv += a.gzp[ct] * nx(ct + 1);
+    wv += a.gxp[ct] * nx(ct + sx);
+    wv += a.gyp[ct] * nx(ct + sy);
+    wn[ct] = wv;
+    rw += r * wv;
+  };
+  double delta = 0.0;
+  if (reason == 0) {  // w = A r
+    cg64_one_pass<ALIGNED, W, true, false>(a, own, words, 0.0, 0.0, rb[0], nullptr, nullptr,
+                                           nullptr, wb[0], nullptr, t0, stride, rr, rw, zz);
+    if (tail) tail_cell(true, false, 0.0, 0.0, rb[0], nullptr, nullptr, nullptr, wb[0], nullptr);
+    double v1[1] = {rw};
+    if (!grid_sum<kCgBlock>(v1, a.part, bid, G, epoch, a.st)) return;
+    delta = v1[0];
+  }
+  double gold = 1.0, al = 1.0, dpi = 0.0, dpiold = 0.0;
+  int i = 0;
+  while (reason == 0) {
+    its = i + 1;
+    if (gamma == 0.0) {
+      reason = 3;
+      break;
+    }
+    if (i > 0 && gamma * gold < 0.0) {
+      reason = -8;
+      break;
+    }
+    const double be = (i == 0) ? 0.0 : gamma / gold;
+    dpiold = dpi;
+    dpi = (i == 0) ? delta : delta - be * gamma / al;
+    if (dpi == 0.0 || (i > 0 && sgn(dpi) * sgn(dpiold) < 0)) {
+      reason = -10;
+      break;
+    }
+    al = gamma / dpi;
+    gold = gamma;
+    const int f = i & 1;
+    rr = rw = zz = 0.0;
+    if (i == 0)
+      cg64_one_pass<ALIGNED, W, false, true>(a, own, words, al, be, rb[f], wb[f], sb[f], rb[1 - f],
+                                             wb[1 - f], sb[1 - f], t0, stride, rr, rw, zz);
+    else
+      cg64_one_pass<ALIGNED, W, false, false>(a, own, words, al, be, rb[f], wb[f], sb[f],
+                                              rb[1 - f], wb[1 - f], sb[1 - f], t0, stride, rr, rw,
+                                              zz);
+    if (tail)
+      tail_cell(false, i == 0, al, be, rb[f], wb[f], sb[f], rb[1 - f], wb[1 - f], sb[1 - f]);
+    double v3[3] = {zz, rr, rw};
+    if (!grid_sum<kCgBlock>(v3, a.part, bid, G, epoch, a.st)) return;
+    dp = sqrt(v3[0]);
+    test(dp);
+    if (reason != 0) break;
+    gamma = v3[1];
+    delta = v3[2];
+    ++i;
+    if (i >= a.maxit) {
+      reason = -3;
+      break;
+    }
+  }
+  o = threadIdx.x;
+  for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
+    const long long c = 2 * q;
+    const double2 s = W > kOneS ? own[kOneS * words + o] : ldp<ALIGNED>(a.z + c);
+    const double2 y = own[kOneY * words + o];
+    stp<ALIGNED>(a.x + c, s.x * y.x, s.y * y.y);
+  }
+  if (tail) a.x[ct] = ts * ty;
+  if (bid == 0 && threadIdx.x == 0) {
+    a.st->dp = dp;
+    a.st->rnorm0 = rnorm0;
+    a.st->its = its;
+    a.st->reason = reason;
+    a.st->outer = 1;
+  }
+}
+
 // 128 registers a thread: at an 80-register cap (768 threads per SM) the
 // kernel spilled and the 512x512x128 FP64 solve took 251 ms against 236.
 template <bool ALIGNED, int W>
 __global__ void __launch_bounds__(kCgBlock, 1) k_cg64(Cg64Args a, int words) {
   extern __shared__ double2 own[];
   cg64v_body<ALIGNED, W>(a, blockIdx.x, gridDim.x, own, words);
+}
+
+template <bool ALIGNED, int W>
+__global__ void __launch_bounds__(kCgBlock, 1) k_cg64_one(Cg64Args a, int words) {
+  extern __shared__ double2 own[];
+  cg64_one_body<ALIGNED, W>(a, blockIdx.x, gridDim.x, own, words);
 }
 
 // One cooperative launch over several domains: instance i owns
@@ -430,6 +706,7 @@ Cg64Args make_cg64_args(const Device& D, double rtol, double atol, int maxit) {
   a.gyp = D.gyp;
   a.gzp = D.gzp;
   a.b = D.rhs;
+  a.bw = D.rhs;
   a.x = D.x;
   a.r = D.r;
   a.z = D.z;
@@ -459,7 +736,20 @@ int cg64_words(long long pairs) {
   return fit >= 7 ? 7 : fit >= 4 ? 4 : fit >= 2 ? 2 : fit >= 1 ? 1 : 0;
 }
 
+// Solves at least this loose, of at most this many pairs a thread on more than
+// one block, take one barrier an iteration; beyond, the third vector's traffic
+// outweighs the barrier (us an iteration, two barriers against one: 48x48x100
+// 8.6 / 6.9, 97x61x75 14.4 / 13.3, 80x80x128 with six pairs 13.4 / 12.8, 81x80x127
+// with six 18.4 / 18.8, 90x90x128 with eight 15.6 / 17.2).
+constexpr double kOneBarrierRtol = 1.0e-10;
+constexpr long long kOneBarrierPairs = 5;
+
 using Cg64Kernel = void (*)(Cg64Args, int);
+template <bool ALIGNED>
+Cg64Kernel cg64_one_kernel(int w) {
+  return w == 7 ? k_cg64_one<ALIGNED, 7> : w == 4 ? k_cg64_one<ALIGNED, 4>
+                                                  : k_cg64_one<ALIGNED, 2>;
+}
 template <bool ALIGNED>
 Cg64Kernel cg64_kernel(int w) {
   return w == 7 ? k_cg64<ALIGNED, 7> : w == 4 ? k_cg64<ALIGNED, 4> : w == 2 ? k_cg64<ALIGNED, 2>
@@ -476,8 +766,11 @@ cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool cle
   const int w = cg64_words(pairs);
   int words = static_cast<int>(pairs * kCgBlock);
   const size_t smem = w * words * sizeof(double2);
-  const void* kern = reinterpret_cast<const void*>((D.d.nz % 2 == 0) ? cg64_kernel<true>(w)
-                                                                     : cg64_kernel<false>(w));
+  const bool even = D.d.nz % 2 == 0, one = w >= 2 && pairs <= kOneBarrierPairs &&
+                                         D.cg_grid > 1 && rtol >= kOneBarrierRtol;
+  const Cg64Kernel k = one ? (even ? cg64_one_kernel<true>(w) : cg64_one_kernel<false>(w))
+                           : (even ? cg64_kernel<true>(w) : cg64_kernel<false>(w));
+  const void* kern = reinterpret_cast<const void*>(k);
   const cudaError_t e = raise_smem_limit(kern, smem);
   if (e != cudaSuccess) return e;
   void* args[] = {&a, &words};
