@@ -68,12 +68,14 @@ cudaError_t dalloc(fgw::Device& D, T** p, size_t n) {
   return cudaSuccess;
 }
 
-// Solver arrays carry a zero margin of one j-row on both ends.
+// Solver arrays carry a zero margin of one j-row on both ends, rounded up so
+// that cell 0 is 16-byte aligned.
 template <class T>
 cudaError_t dalloc_margin(fgw::Device& D, T** p, long long ncell, long long margin) {
   T* base = nullptr;
-  cudaError_t e = dalloc(D, &base, static_cast<size_t>(ncell + 2 * margin));
-  *p = base ? base + margin : nullptr;
+  const long long m = static_cast<long long>(fgw::solve_margin(margin));
+  cudaError_t e = dalloc(D, &base, static_cast<size_t>(ncell + 2 * m));
+  *p = base ? base + m : nullptr;
   return e;
 }
 

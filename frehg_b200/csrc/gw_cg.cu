@@ -21,7 +21,7 @@
 //   phase B: r -= a w, partials r'r and ||S r||^2 = ||D^-1 r||^2 (unscaled);
 //   the same barrier; convergence test.
 // Every thread takes two consecutive cells (cg64v_body), with 16-byte pair
-// loads where nz is even and separate loads where it is odd.
+// loads (ld_far for the neighbours' pairs where nz is odd).
 // Per cell and iteration this moves 12.5 FP64 words (100 B): phase A reads r,
 // p_old, gxp, gyp, gzp and writes p_new, w, and half the time reads y and the
 // p before p_old (in p_new's buffer) and writes y; phase B reads r, w, s and
@@ -72,32 +72,24 @@ constexpr long long kCgAlone = 2 * kCgBlock;
 
 __device__ inline int sgn(double v) { return (v > 0.0) - (v < 0.0); }
 
-// Two consecutive cells per thread.  With ALIGNED (nz even, so every pair and
-// every i/j-neighbour pair is 16-byte aligned) the pairs move as 16-byte loads
-// and stores: half the load instructions per cell and twice the bytes in
-// flight per request.  Otherwise (nz odd) the pair's two cells load
-// separately, still two cells' loads in flight per thread, and an odd cell
-// count leaves a last cell that one thread takes alone (cg64_cell_*).
+// Two consecutive cells per thread, moved as 16-byte pairs: cell 0 of every
+// array is 16-byte aligned, so a thread's own pairs are.  Its i and j
+// neighbours' are with ALIGNED (nz even); otherwise see ld_far, and an odd
+// cell count leaves a last cell that one thread takes alone (cg64_cell_*).
 __device__ inline double2 ld2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 __device__ inline void st2(double* p, double a, double b) {
   *reinterpret_cast<double2*>(p) = make_double2(a, b);
 }
+// Pairs a whole number of columns away from a thread's own: with nz odd they
+// may start on an odd cell and are two loads, without asking (a branch on the
+// parity took a 256x256x127 iteration from 160 to 204 us: it parts the loads).
+// One aligned load and a shuffle from the lane before would halve the loads,
+// but a shuffle holds up the loads behind it: 436 us.  With a thread's own
+// pairs as two loads as well it was 247 us.
 template <bool ALIGNED>
-__device__ inline double2 ldp(const double* p) {
-  if constexpr (ALIGNED) {
-    return ld2(p);
-  } else {
-    return make_double2(p[0], p[1]);
-  }
-}
-template <bool ALIGNED>
-__device__ inline void stp(double* p, double a, double b) {
-  if constexpr (ALIGNED) {
-    st2(p, a, b);
-  } else {
-    p[0] = a;
-    p[1] = b;
-  }
+__device__ inline double2 ld_far(const double* p) {
+  if (ALIGNED) return ld2(p);
+  return make_double2(p[0], p[1]);
 }
 
 // The steps of one cell alone (the order of terms of the pair code), for the
@@ -165,29 +157,29 @@ __device__ __forceinline__ double cg64_phase_a(const Cg64Args& a, double2* __res
     const auto chip = [&](int word) -> double2& { return own[word * words + o]; };
     const auto leg = [&](int word, const double* g) {
       if (W > word && !FIRST) return chip(word);
-      const double2 v = ldp<ALIGNED>(g);
+      const double2 v = ld_far<ALIGNED>(g);
       if (W > word) chip(word) = v;
       return v;
     };
     const double2 zero = make_double2(0.0, 0.0);
-    const double2 rc = ldp<ALIGNED>(r + c);
-    const double2 pc = FIRST ? zero : ldp<ALIGNED>(pold + c);
-    const double2 rxm = ldp<ALIGNED>(r + c - sx), rxp = ldp<ALIGNED>(r + c + sx);
-    const double2 rym = ldp<ALIGNED>(r + c - sy), ryp = ldp<ALIGNED>(r + c + sy);
-    const double2 pxm = FIRST ? zero : ldp<ALIGNED>(pold + c - sx);
-    const double2 pxp = FIRST ? zero : ldp<ALIGNED>(pold + c + sx);
-    const double2 pym = FIRST ? zero : ldp<ALIGNED>(pold + c - sy);
-    const double2 pyp = FIRST ? zero : ldp<ALIGNED>(pold + c + sy);
+    const double2 rc = ld2(r + c);
+    const double2 pc = FIRST ? zero : ld2(pold + c);
+    const double2 rxm = ld_far<ALIGNED>(r + c - sx), rxp = ld_far<ALIGNED>(r + c + sx);
+    const double2 rym = ld_far<ALIGNED>(r + c - sy), ryp = ld_far<ALIGNED>(r + c + sy);
+    const double2 pxm = FIRST ? zero : ld_far<ALIGNED>(pold + c - sx);
+    const double2 pxp = FIRST ? zero : ld_far<ALIGNED>(pold + c + sx);
+    const double2 pym = FIRST ? zero : ld_far<ALIGNED>(pold + c - sy);
+    const double2 pyp = FIRST ? zero : ld_far<ALIGNED>(pold + c + sy);
     const double rkm = r[c - 1], rkp = r[c + 2];
     const double pkm = FIRST ? 0.0 : pold[c - 1], pkp = FIRST ? 0.0 : pold[c + 2];
     const double2 gx = leg(kOwnGx, gxp + c), gxm = leg(kOwnGxm, gxp + c - sx);
     const double2 gy = leg(kOwnGy, gyp + c), gym = leg(kOwnGym, gyp + c - sy);
-    const double2 gz = ldp<ALIGNED>(gzp + c);
+    const double2 gz = ld2(gzp + c);
     const double gzm = gzp[c - 1];
     double2 y = zero, pp = zero;
     if (YUP) {
-      y = W > kOwnY ? chip(kOwnY) : ldp<ALIGNED>(x + c);
-      pp = ldp<ALIGNED>(pnew + c);
+      y = W > kOwnY ? chip(kOwnY) : ld2(x + c);
+      pp = ld2(pnew + c);
     }
     const double P0 = rc.x + bc * pc.x, P1 = rc.y + bc * pc.y;
     double w0 = gym.x * (rym.x + bc * pym.x);
@@ -204,14 +196,14 @@ __device__ __forceinline__ double cg64_phase_a(const Cg64Args& a, double2* __res
     w1 += gz.y * (rkp + bc * pkp);
     w1 += gx.y * (rxp.y + bc * pxp.y);
     w1 += gy.y * (ryp.y + bc * pyp.y);
-    stp<ALIGNED>(pnew + c, P0, P1);
+    st2(pnew + c, P0, P1);
     if (W > kOwnW) chip(kOwnW) = make_double2(w0, w1);
-    else stp<ALIGNED>(w + c, w0, w1);
+    else st2(w + c, w0, w1);
     if (YUP) {
       y.x += al1 * pc.x + al2 * pp.x;
       y.y += al1 * pc.y + al2 * pp.y;
       if (W > kOwnY) chip(kOwnY) = y;
-      else stp<ALIGNED>(x + c, y.x, y.y);
+      else st2(x + c, y.x, y.y);
     }
     pw += P0 * w0;
     pw += P1 * w1;
@@ -241,22 +233,22 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   int o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
-    const double2 bv = ldp<ALIGNED>(b + c), dg = ldp<ALIGNED>(diag + c);
-    const double2 dx = ldp<ALIGNED>(diag + c + sx), dy = ldp<ALIGNED>(diag + c + sy);
+    const double2 bv = ld2(b + c), dg = ld2(diag + c);
+    const double2 dx = ld_far<ALIGNED>(diag + c + sx), dy = ld_far<ALIGNED>(diag + c + sy);
     const double dz = diag[c + 2];
-    const double2 gx = ldp<ALIGNED>(gxp + c), gy = ldp<ALIGNED>(gyp + c);
-    const double2 gz = ldp<ALIGNED>(gzp + c);
+    const double2 gx = ld2(gxp + c), gy = ld2(gyp + c);
+    const double2 gz = ld2(gzp + c);
     const double s0 = 1.0 / sqrt(dg.x), s1 = 1.0 / sqrt(dg.y);
     const double r0 = s0 * bv.x, r1 = s1 * bv.y;
-    stp<ALIGNED>(gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
-    stp<ALIGNED>(gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
-    stp<ALIGNED>(gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
-    stp<ALIGNED>(ra + c, r0, r1);
-    stp<ALIGNED>(a.p0 + c, 0.0, 0.0);
+    st2(gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
+    st2(gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
+    st2(gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
+    st2(ra + c, r0, r1);
+    st2(a.p0 + c, 0.0, 0.0);
     if (W > kOwnS) own[kOwnS * words + o] = make_double2(s0, s1);
-    else stp<ALIGNED>(sa + c, s0, s1);
+    else st2(sa + c, s0, s1);
     if (W > kOwnY) own[kOwnY * words + o] = make_double2(0.0, 0.0);
-    else stp<ALIGNED>(xa + c, 0.0, 0.0);
+    else st2(xa + c, 0.0, 0.0);
     const double z0 = s0 * r0, z1 = s1 * r1;
     rr += r0 * r0;
     rr += r1 * r1;
@@ -318,11 +310,11 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     o = threadIdx.x;
     for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
       const long long c = 2 * q;
-      const double2 r = ldp<ALIGNED>(ra + c);
-      const double2 w = W > kOwnW ? own[kOwnW * words + o] : ldp<ALIGNED>(wa + c);
-      const double2 s = W > kOwnS ? own[kOwnS * words + o] : ldp<ALIGNED>(sa + c);
+      const double2 r = ld2(ra + c);
+      const double2 w = W > kOwnW ? own[kOwnW * words + o] : ld2(wa + c);
+      const double2 s = W > kOwnS ? own[kOwnS * words + o] : ld2(sa + c);
       const double r0 = r.x - al * w.x, r1 = r.y - al * w.y;
-      stp<ALIGNED>(ra + c, r0, r1);
+      st2(ra + c, r0, r1);
       const double z0 = s.x * r0, z1 = s.y * r1;
       rr += r0 * r0;
       rr += r1 * r1;
@@ -356,8 +348,8 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
-    const double2 s = W > kOwnS ? own[kOwnS * words + o] : ldp<ALIGNED>(sa + c);
-    const double2 y = W > kOwnY ? own[kOwnY * words + o] : ldp<ALIGNED>(xa + c);
+    const double2 s = W > kOwnS ? own[kOwnS * words + o] : ld2(sa + c);
+    const double2 y = W > kOwnY ? own[kOwnY * words + o] : ld2(xa + c);
     fin(s.x, y.x, c);
     fin(s.y, y.y, c + 1);
   }
@@ -401,20 +393,20 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
     const auto chip = [&](int word) -> double2& { return own[word * words + o]; };
     const auto leg = [&](int word, const double* g) {
       if (W > word && !START) return chip(word);
-      const double2 v = ldp<ALIGNED>(g);
+      const double2 v = ld_far<ALIGNED>(g);
       if (W > word) chip(word) = v;
       return v;
     };
     // r - al (w + be s) of a pair (START: r; FIRST: r - al w)
     const auto next2 = [&](long long m) {
-      double2 r = ldp<ALIGNED>(ro + m);
+      double2 r = ld_far<ALIGNED>(ro + m);
       if (START) return r;
-      const double2 w = ldp<ALIGNED>(wo + m);
+      const double2 w = ld_far<ALIGNED>(wo + m);
       if (FIRST) {
         r.x -= al * w.x;
         r.y -= al * w.y;
       } else {
-        const double2 s = ldp<ALIGNED>(so + m);
+        const double2 s = ld_far<ALIGNED>(so + m);
         r.x -= al * (w.x + be * s.x);
         r.y -= al * (w.y + be * s.y);
       }
@@ -428,14 +420,14 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
     const double rkm = next1(c - 1), rkp = next1(c + 2);
     const double2 gx = leg(kOneGx, a.gxp + c), gxm = leg(kOneGxm, a.gxp + c - sx);
     const double2 gy = leg(kOneGy, a.gyp + c), gym = leg(kOneGym, a.gyp + c - sy);
-    const double2 gz = ldp<ALIGNED>(a.gzp + c);
+    const double2 gz = ld2(a.gzp + c);
     const double gzm = a.gzp[c - 1];
-    double2 r = ldp<ALIGNED>(ro + c);
+    double2 r = ld2(ro + c);
     if (!START) {
-      double2 s = ldp<ALIGNED>(wo + c), p = r;
+      double2 s = ld2(wo + c), p = r;
       double2 y = make_double2(0.0, 0.0);
       if (!FIRST) {
-        const double2 sp = ldp<ALIGNED>(so + c), pp = chip(kOneP);
+        const double2 sp = ld2(so + c), pp = chip(kOneP);
         y = chip(kOneY);
         s.x += be * sp.x;
         s.y += be * sp.y;
@@ -448,9 +440,9 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
       chip(kOneY) = y;
       r.x -= al * s.x;
       r.y -= al * s.y;
-      stp<ALIGNED>(rn + c, r.x, r.y);
-      stp<ALIGNED>(sn + c, s.x, s.y);
-      const double2 S = W > kOneS ? chip(kOneS) : ldp<ALIGNED>(a.z + c);
+      st2(rn + c, r.x, r.y);
+      st2(sn + c, s.x, s.y);
+      const double2 S = W > kOneS ? chip(kOneS) : ld2(a.z + c);
       const double z0 = S.x * r.x, z1 = S.y * r.y;
       rr += r.x * r.x;
       rr += r.y * r.y;
@@ -471,7 +463,7 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
     w1 += gz.y * rkp;
     w1 += gx.y * rxp.y;
     w1 += gy.y * ryp.y;
-    stp<ALIGNED>(wn + c, w0, w1);
+    st2(wn + c, w0, w1);
     rw += r.x * w0;
     rw += r.y * w1;
   }
@@ -496,19 +488,19 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
   int o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
-    const double2 bv = ldp<ALIGNED>(a.b + c), dg = ldp<ALIGNED>(a.diag + c);
-    const double2 dx = ldp<ALIGNED>(a.diag + c + sx), dy = ldp<ALIGNED>(a.diag + c + sy);
+    const double2 bv = ld2(a.b + c), dg = ld2(a.diag + c);
+    const double2 dx = ld_far<ALIGNED>(a.diag + c + sx), dy = ld_far<ALIGNED>(a.diag + c + sy);
     const double dz = a.diag[c + 2];
-    const double2 gx = ldp<ALIGNED>(a.gxp + c), gy = ldp<ALIGNED>(a.gyp + c);
-    const double2 gz = ldp<ALIGNED>(a.gzp + c);
+    const double2 gx = ld2(a.gxp + c), gy = ld2(a.gyp + c);
+    const double2 gz = ld2(a.gzp + c);
     const double s0 = 1.0 / sqrt(dg.x), s1 = 1.0 / sqrt(dg.y);
     const double r0 = s0 * bv.x, r1 = s1 * bv.y;
-    stp<ALIGNED>(a.gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
-    stp<ALIGNED>(a.gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
-    stp<ALIGNED>(a.gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
-    stp<ALIGNED>(a.r + c, r0, r1);
+    st2(a.gxp + c, gx.x * (s0 / sqrt(dx.x)), gx.y * (s1 / sqrt(dx.y)));
+    st2(a.gyp + c, gy.x * (s0 / sqrt(dy.x)), gy.y * (s1 / sqrt(dy.y)));
+    st2(a.gzp + c, gz.x * (s0 * s1), gz.y * (s1 / sqrt(dz)));
+    st2(a.r + c, r0, r1);
     if (W > kOneS) own[kOneS * words + o] = make_double2(s0, s1);
-    else stp<ALIGNED>(a.z + c, s0, s1);
+    else st2(a.z + c, s0, s1);
     const double z0 = s0 * r0, z1 = s1 * r1;
     rr += r0 * r0;
     rr += r1 * r1;
@@ -623,9 +615,9 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
   o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
-    const double2 s = W > kOneS ? own[kOneS * words + o] : ldp<ALIGNED>(a.z + c);
+    const double2 s = W > kOneS ? own[kOneS * words + o] : ld2(a.z + c);
     const double2 y = own[kOneY * words + o];
-    stp<ALIGNED>(a.x + c, s.x * y.x, s.y * y.y);
+    st2(a.x + c, s.x * y.x, s.y * y.y);
   }
   if (tail) a.x[ct] = ts * ty;
   if (bid == 0 && threadIdx.x == 0) {

@@ -61,6 +61,9 @@ enum PartialSlot {
 // reduction has the same shape, and therefore the same rounding, each step).
 constexpr int kBlock = 256;
 
+// Cells of margin a solve vector takes for a j-row of them.
+inline size_t solve_margin(size_t row) { return (row + 3) & ~static_cast<size_t>(3); }
+
 // Reduction slots (doubles) a solve block needs (coop::grid_sum).
 constexpr size_t kSolveSlots = 8;
 

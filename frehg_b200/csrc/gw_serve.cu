@@ -247,7 +247,7 @@ size_t frehg_gw_device_bytes(const frehg_gw_desc* d) {
   // SMs, so the figure holds for any device.
   const size_t ncol = static_cast<size_t>(d->nx + 2) * (d->ny + 2);
   const size_t n3 = ncol * d->nz, nf = ncol * (d->nz + 1);
-  const size_t m = static_cast<size_t>(d->nx + 2) * d->nz, ns = n3 + 2 * m;
+  const size_t m = static_cast<size_t>(d->nx + 2) * d->nz, ns = n3 + 2 * fgw::solve_margin(m);
   auto r = [](size_t bytes) { return (bytes + 255) & ~static_cast<size_t>(255); };
   int arrays = 8, ones = 0;  // geometry; soil by fgw::soil_storage
   for (int f = 0; f < 8; ++f) {
