@@ -220,33 +220,32 @@ struct LineSolve {
 #pragma unroll
     for (int e = 0; e < E; ++e) zr += static_cast<double>(zv[e]) * static_cast<double>(r[e]);
   }
-  __device__ static __forceinline__ void solve_deep(const LineArgs<T>& a, int base, double& zr) {
+  // The chunked column's solve: the forward sweep chunk by chunk as r is made
+  // (y through z, its last value carried; z'r = y'y), then the backward one.
+  __device__ static __forceinline__ void deep_forward(const LineArgs<T>& a, const Place& p,
+                                                      const T (&r)[E], T& carry, double& zr) {
+    T l[E], y[E];
+    ld_cells<E>(a.v.l + p.cp + p.k0, p.n, l);
+    T lm = __shfl_up_sync(kFull, l[E - 1], 1, LPC);
+    if (p.q == 0) lm = p.k0 > 0 ? a.v.l[p.cp + p.k0 - 1] : T(0);
+    line_forward<LPC, E>(l, lm, r, carry, p.q, y);
+    st_cells<E>(a.v.z + p.cp + p.k0, p.n, y);
+    carry = __shfl_sync(kFull, y[E - 1], LPC - 1, LPC);
+#pragma unroll
+    for (int e = 0; e < E; ++e) zr += static_cast<double>(y[e]) * static_cast<double>(y[e]);
+  }
+  __device__ static __forceinline__ void deep_backward(const LineArgs<T>& a, int base) {
     const int nzp = line_nzp(a.d.nz), chunk = LPC * E;
     T carry = T(0);
-    Place p;
-    for (int kb = 0; kb < nzp; kb += chunk) {  // y into z
-      place(a, base, kb, p);
-      T l[E], r[E], y[E];
-      ld_cells<E>(a.v.l + p.cp + p.k0, p.n, l);
-      ld_cells<E>(a.v.r + p.cp + p.k0, p.n, r);
-      T lm = __shfl_up_sync(kFull, l[E - 1], 1, LPC);
-      if (p.q == 0) lm = kb > 0 ? a.v.l[p.cp + kb - 1] : T(0);
-      line_forward<LPC, E>(l, lm, r, carry, p.q, y);
-      st_cells<E>(a.v.z + p.cp + p.k0, p.n, y);
-      carry = __shfl_sync(kFull, y[E - 1], LPC - 1, LPC);
-    }
-    carry = T(0);
     for (int kb = (nzp - 1) / chunk * chunk; kb >= 0; kb -= chunk) {
+      Place p;
       place(a, base, kb, p);
-      T l[E], r[E], y[E], z[E];
+      T l[E], y[E], z[E];
       ld_cells<E>(a.v.l + p.cp + p.k0, p.n, l);
-      ld_cells<E>(a.v.r + p.cp + p.k0, p.n, r);
       ld_cells<E>(a.v.z + p.cp + p.k0, p.n, y);
       line_backward<LPC, E>(l, y, carry, p.q, z);
       st_cells<E>(a.v.z + p.cp + p.k0, p.n, z);
       carry = __shfl_sync(kFull, z[0], 0, LPC);
-#pragma unroll
-      for (int e = 0; e < E; ++e) zr += static_cast<double>(z[e]) * static_cast<double>(r[e]);
     }
   }
 
@@ -265,6 +264,7 @@ struct LineSolve {
                  *const gzp = a.gzp;
     int m = 0;
     for (int base = gwarp * kCols; base < d.nx * d.ny; base += nwarp * kCols, ++m) {
+      T carry = T(0);
       for (int kb = 0; kb < (DEEP ? nzp : 1); kb += LPC * E) {
         Place p;
         place(a, base, kb, p);
@@ -342,12 +342,11 @@ struct LineSolve {
           T l[E];
           ld_leg<kLineL>(own, m, FIRST, a.v.l + cp + k0, n, l);
           solve_store(a.v.z, l, r, p, zr);
+        } else {
+          deep_forward(a, p, r, carry, zr);
         }
       }
-      if (DEEP) {
-        __syncwarp();
-        solve_deep(a, base, zr);
-      }
+      if (DEEP) deep_backward(a, base);
     }
   }
 
@@ -454,6 +453,7 @@ struct LineSolve {
     int m = 0;
     for (int base = gwarp * kCols; base < ncols; base += kPassB * step, m += kPassB) {
       if constexpr (DEEP) {
+        T carry = T(0);
         for (int kb = 0; kb < nzp; kb += LPC * E) {
           Place p;
           place(a, base, kb, p);
@@ -464,9 +464,9 @@ struct LineSolve {
 #pragma unroll
           for (int e = 0; e < E; ++e) r[e] -= al * w[e];
           st_cells<E>(rv + c, p.n, r);
+          deep_forward(a, p, r, carry, zr);
         }
-        __syncwarp();
-        solve_deep(a, base, zr);
+        deep_backward(a, base);
       } else {
         Place p[kPassB];
         T w[kPassB][E], r[kPassB][E], l[kPassB][E];
