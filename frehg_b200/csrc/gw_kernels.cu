@@ -2457,8 +2457,11 @@ void launch_update_wc(const Device& D, const double* hn, const double* wcn) {
 }
 
 // Columns up to kWalkMaxNz cells take the warp walk (dynamic shared memory
-// opted in up to kWalkSmemMax); deeper columns take the per-thread walk.
-constexpr int kWalkMaxNz = 256;
+// opted in up to kWalkSmemMax, two blocks per SM at the deepest); deeper
+// columns take the per-thread walk, whose one thread a column is all latency:
+// the post-allocation of a 24x20x300 hillslope takes 5.3 ms with it, 0.13 with
+// the warp walk.
+constexpr int kWalkMaxNz = 352;
 constexpr size_t kWalkSmemMax = 96 * 1024;
 
 bool warp_walk(const Device& D) {

@@ -372,7 +372,7 @@ typedef struct frehg_gw_batch frehg_gw_batch;
 
 typedef struct {
   int cells_per_block;  /* active cells per solve block of a member; 0 = 16384 */
-  int tiled_line_solve; /* mixed form: 1 = shared-memory tiled line solve at every depth */
+  int tiled_line_solve; /* mixed form: 1 = columns in chunks at every depth (the deep columns' form) */
   int use_graph;        /* 1 = replay each step as a CUDA graph, 0 = launch directly */
   int streams;          /* per_member_phases: concurrent member streams; 0 = 32 */
   int per_member_phases;/* 1 = launch each member's non-solve kernels on its own (streams);
@@ -410,7 +410,7 @@ int frehg_gw_batch_step(frehg_gw_batch* b, frehg_gw_step_info* infos);
 /* Overrides member i's dt for the next batch step (e.g. to end on a time). */
 int frehg_gw_batch_set_dt(frehg_gw_batch* b, int i, double dtg);
 /* Times candidate decompositions (solve blocks per member, and for the mixed
- * form the column or tiled line solve) on trial steps from a snapshot of the
+ * form whole or chunked columns) on trial steps from a snapshot of the
  * members' state, restores that state and keeps the fastest; results are
  * cached per batch shape for the process.  best_ms is -1 on a cache hit.
  * Candidates: 4096..131072 cells per block. */
