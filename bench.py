@@ -44,15 +44,15 @@ sys.path.insert(0, ROOT)
 
 # Algorithmic bytes per active cell (interior cells, each array read or
 # written once per pass).
-ALG_BYTES_PER_CG_ITER = 128   # FP64 Jacobi-PCG iteration: 16 words
-ALG_BYTES_MIXED_INNER = 64    # FP32 inner iteration: stencil pass 10 words (z, p_old,
-                              # d, diag, gxp, gyp, gzp in; p, w, d out; d += alpha p of
-                              # the previous iteration), update + line solve 6 words
-                              # (r, w, dinv, l in; r, z out)
+ALG_BYTES_PER_CG_ITER = 100   # FP64 Jacobi-PCG iteration: 12.5 words
+ALG_BYTES_MIXED_INNER = 54    # FP32 inner iteration: stencil pass 8.5 words (z, p_old,
+                              # gx, gy, l in; p, w out; every second iteration d and
+                              # the p before in, d out), update + line solve 5 words
+                              # (r, w, l in; r, z out)
 ALG_BYTES_MIXED_FIRST = 12    # less in each inner solve's first iteration (p = z:
                               # neither p_old nor d)
 ALG_BYTES_MIXED_SWEEP = 76    # FP64 outer residual sweep: x, b, 4 coefficients, d, l,
-                              # dinv in; x, r, z out
+                              # scale in; x, r, z out
 ALG_BYTES_MIXED_OUTER = 8     # per correction: its last update's p, read by the next
                               # sweep, and the d reset
 ALG_BYTES_MIXED_INIT = 12     # b read for ||b||, d = 0 at entry (the assembly writes
@@ -62,7 +62,7 @@ METRIC = "cell-steps/s at 512x512x128"
 # DRAM bytes (read + write) per algorithmic byte of k_cg_mixed, from the ncu
 # capture summarised in profiles/ (256x256x128 slab, one steady-state launch);
 # scaled to the timed launches by their algorithmic bytes.
-MIXED_TRAFFIC_PER_ALG_BYTE = 1.023
+MIXED_TRAFFIC_PER_ALG_BYTE = 1.020
 # Bytes frehg_gw_step reads back per step: the device step record (nine FP64
 # audit and controller terms, the solver's exit state, the coupled-top books).
 STEP_RECORD_BYTES = 192
@@ -628,7 +628,7 @@ def main():
                 (fp64["solve_ms"] / 1e3) / 1e9) if fp64["solve_ms"] else 0.0
     mixed_ach = (mixed_alg_bytes(mixed["active"], mixed["iters"], mixed["outer"], args.steps) /
                  (mixed["solve_ms"] / 1e3) / 1e9) if mixed["solve_ms"] else 0.0
-    roof_fp64 = {"bound": "hbm", "kernel": "k_cg64v (FP64 Jacobi-PCG, one launch per step)",
+    roof_fp64 = {"bound": "hbm", "kernel": "k_cg64 (FP64 Jacobi-PCG, one launch per step)",
                  "achieved": fp64_ach, "peak": peak, "unit": "GB/s", "frac": fp64_ach / peak,
                  "peak_source": peak_kind, "alg_bytes_per_cell_iter": ALG_BYTES_PER_CG_ITER,
                  "cg_iterations_per_step": fp64["iters"] / args.steps,
@@ -662,7 +662,7 @@ def main():
                       "inner_iterations_per_step": res_line["iters"] / args.steps,
                       "outer_sweeps_per_step": res_line["outer"] / args.steps,
                       "solve_ms_per_step": res_line["solve_ms"] / args.steps,
-                      "solve_alg_bytes_per_cell_inner": 128,
+                      "solve_alg_bytes_per_cell_inner": 108,
                       "latency": res_line["latency"]},
         "mixed_over_fp64": mixed["value"] / fp64["value"] if fp64["value"] else None,
         # the split of mixed / FP64: precision alone (same algorithm, FP64

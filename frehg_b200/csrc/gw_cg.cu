@@ -35,7 +35,7 @@
 // A thread's cells stay its own for the whole solve, so the words only it
 // reads can stay in shared memory (cg64_words: as many of w, y, s and the legs
 // as the domain's size leaves room for).  512x512x128 (no room) 692 -> 571 us an
-// iteration, 131x113x127 (w) 48.2 -> 36.7, 64x64x128 (four) 12.7 -> 11.0.
+// iteration, 131x113x127 (w) 48.2 -> 35.8, 64x64x128 (four) 12.7 -> 11.0.
 //
 // The grid barrier's wait is bounded: one that exceeds kSpinLimit polls sets
 // CgState::err, and every block leaves at its next barrier, so a launch that

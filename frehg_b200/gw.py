@@ -295,7 +295,7 @@ class RichardsSolver:
         _check(self.lib, self.lib.frehg_gw_set_profiling(self.h, int(bool(on))))
 
     def setFused(self, on: bool = True) -> None:
-        """Fused phase kernels (default) or every phase as separate passes."""
+        """Every phase as separate passes (off, the only form); on is refused."""
         _check(self.lib, self.lib.frehg_gw_set_fused(self.h, int(bool(on))))
 
     def setWarmStart(self, extrapolate: bool = True) -> None:

@@ -263,13 +263,10 @@ int frehg_gw_device(const frehg_gw_handle* h);
 int frehg_gw_set_profiling(frehg_gw_handle* h, int on);
 int frehg_gw_phase_times(frehg_gw_handle* h, double* ms5);
 
-/* Kernel selection (no counterpart in the reference).  The fused predictor
- * (closures, faces, rows and the mixed form's column factors in one pass) and
- * fused corrector (head scatter, closures, faces, fluxes, theta update) for
- * groundwater-only domains with nz <= 256 raised a misaligned-address error
- * on the B200 whose cause is not yet found, so they are disabled: on = 1
- * returns FREHG_GW_EUNSUPPORTED, on = 0 (every phase as its separate passes,
- * the default) succeeds. */
+/* Kernel selection (no counterpart in the reference).  Fused predictor and
+ * corrector passes raised a misaligned-address error on the B200 and were
+ * taken out: on = 1 returns FREHG_GW_EUNSUPPORTED, on = 0 (every phase as its
+ * separate passes, the default) succeeds. */
 int frehg_gw_set_fused(frehg_gw_handle* h, int on);
 
 /* Starting iterate of the mixed and FP64 line solves (no counterpart in the
