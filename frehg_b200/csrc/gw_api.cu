@@ -561,7 +561,11 @@ int frehg_gw_init_state(frehg_gw_handle* h, int form, double constant, const dou
                          ? static_cast<size_t>(d.nx) * d.ny
                          : static_cast<size_t>(d.nx) * d.ny * d.nz;
     CUDA_TRY(cudaMalloc(&fdev, n * sizeof(double)), "init_state");
-    CUDA_TRY(cudaMemcpy(fdev, field, n * sizeof(double), cudaMemcpyHostToDevice), "init_state");
+    // On the domain's stream, as every upload its kernels read: a plain copy
+    // from pageable memory returns with its last part still in flight, and
+    // the (non-blocking) stream does not wait for it.
+    CUDA_TRY(cudaMemcpyAsync(fdev, field, n * sizeof(double), cudaMemcpyHostToDevice, D.stream),
+             "init_state");
   }
   D.cur = 0;
   fgw::launch_init_state(D, form, constant, fdev, h->bath_dev, h->offset);
@@ -598,10 +602,10 @@ int frehg_gw_set_state(frehg_gw_handle* h, const double* head, const double* wc)
       }
   if (D.f.baro) fgw::launch_baro(D);  // refreshDerivedState (RichardsSolver.cpp:880-890)
   for (int b = 0; b < 2; ++b) {
-    CUDA_TRY(cudaMemcpy(D.h[b], hh.data(), d.ncell * sizeof(double), cudaMemcpyHostToDevice),
-             "set_state");
-    CUDA_TRY(cudaMemcpy(D.wc[b], ww.data(), d.ncell * sizeof(double), cudaMemcpyHostToDevice),
-             "set_state");
+    CUDA_TRY(cudaMemcpyAsync(D.h[b], hh.data(), d.ncell * sizeof(double), cudaMemcpyHostToDevice,
+                             D.stream), "set_state");
+    CUDA_TRY(cudaMemcpyAsync(D.wc[b], ww.data(), d.ncell * sizeof(double), cudaMemcpyHostToDevice,
+                             D.stream), "set_state");
     fgw::launch_ghosts(D, D.h[b], D.wc[b]);
   }
   CUDA_TRY(cudaStreamSynchronize(D.stream), "set_state");
@@ -627,8 +631,9 @@ int frehg_gw_restore(frehg_gw_handle* h, const double* head, const double* wc,
         for (int k = 0; k < d.nz; ++k)
           v[fgw::cidx(d, j, i, k)] =
               vloss[(static_cast<long long>(j - 1) * d.nx + (i - 1)) * d.nz + k];
-    CUDA_TRY(cudaMemcpy(D.vloss, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice),
-             "restore");
+    CUDA_TRY(cudaMemcpyAsync(D.vloss, v.data(), v.size() * sizeof(double), cudaMemcpyHostToDevice,
+                             D.stream), "restore");
+    CUDA_TRY(cudaStreamSynchronize(D.stream), "restore");
   }
   h->next_dt = dtg;
   return FREHG_GW_OK;
@@ -1006,8 +1011,9 @@ int frehg_gw_restore_prev(frehg_gw_handle* h, const double* head_prev, double pr
   for (int j = 1; j <= d.ny; ++j)
     for (int i = 1; i <= d.nx; ++i)
       for (int k = 0; k < d.nz; ++k) full[fgw::cidx(d, j, i, k)] = head_prev[q++];
-  CUDA_TRY(cudaMemcpy(D.h[1 - D.cur], full.data(), full.size() * sizeof(double),
-                      cudaMemcpyHostToDevice), "restore_prev");
+  CUDA_TRY(cudaMemcpyAsync(D.h[1 - D.cur], full.data(), full.size() * sizeof(double),
+                           cudaMemcpyHostToDevice, D.stream), "restore_prev");
+  CUDA_TRY(cudaStreamSynchronize(D.stream), "restore_prev");
   h->have_prev = true;
   h->prev_dtg = prev_dt;
   return FREHG_GW_OK;

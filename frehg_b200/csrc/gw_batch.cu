@@ -164,7 +164,8 @@ size_t solve_group_bytes(const SolveClass& c, int n) {
 
 cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vector<Device*>& ds,
                               const std::vector<int>& variants, const std::vector<int>& nb,
-                              const std::vector<SolveParams>& p, int max_grid, void* mem) {
+                              const std::vector<SolveParams>& p, int max_grid, void* mem,
+                              cudaStream_t s) {
   g.cls = c;
   g.n = static_cast<int>(ds.size());
   const size_t ab = args_bytes(c);
@@ -193,13 +194,17 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   g.queue = reinterpret_cast<int*>(q);
   g.order = reinterpret_cast<int*>(q + r(sizeof(int)));
   g.ofirst = reinterpret_cast<int*>(q + r(sizeof(int)) + r(sizeof(int) * ds.size()));
-  cudaError_t e = cudaMemcpy(g.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMemcpyAsync(g.tab, tab.data(), tab.size(), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
-    e = cudaMemcpy(g.first, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(g.first, first.data(), first.size() * sizeof(int),
+                        cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
-    e = cudaMemcpy(g.states, st.data(), st.size() * sizeof(CgState*), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(g.states, st.data(), st.size() * sizeof(CgState*),
+                        cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess)
-    e = cudaMemcpy(g.parts, parts.data(), parts.size() * sizeof(double*), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(g.parts, parts.data(), parts.size() * sizeof(double*),
+                        cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e;
 }
 
@@ -322,7 +327,8 @@ int build_groups(frehg_gw_batch* b) {
   for (const auto& sp : specs) {
     fgw::SolveGroup g;
     const cudaError_t e = fgw::solve_group_build(g, sp.c, sp.ds, sp.variants, sp.nbs, sp.ps,
-                                                 sp.cap, static_cast<char*>(b->group_mem) + off);
+                                                 sp.cap, static_cast<char*>(b->group_mem) + off,
+                                                 b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch: solve group");
     off += fgw::solve_group_bytes(sp.c, static_cast<int>(sp.ds.size()));
     b->groups.push_back(g);
@@ -414,7 +420,7 @@ int build_member_tables(frehg_gw_batch* b) {
     ds.push_back(&h->D);
     mixed.push_back(h->precision == FREHG_GW_PRECISION_MIXED ? 1 : 0);
   }
-  const cudaError_t ep = fgw::phase_tables_build(b->phases, ds, mixed);
+  const cudaError_t ep = fgw::phase_tables_build(b->phases, ds, mixed, b->stream);
   return ep == cudaSuccess ? FREHG_GW_OK : cuda_fail(ep, "batch: phase tables");
 }
 

@@ -267,9 +267,9 @@ int frehg_gw_set_scalar(frehg_gw_handle* h, int which, const double* values) {
   if (!values) return fail(FREHG_GW_EINVAL, "set_scalar: null values");
   fgw::Device& D = h->D;
   const size_t n = static_cast<size_t>(cell_scalar(which) ? D.d.ncell : D.d.ncol);
+  CUDA_TRY(cudaMemcpyAsync(D.scal[which], values, n * sizeof(double), cudaMemcpyHostToDevice,
+                           D.stream), "set_scalar");
   CUDA_TRY(cudaStreamSynchronize(D.stream), "set_scalar");
-  CUDA_TRY(cudaMemcpy(D.scal[which], values, n * sizeof(double), cudaMemcpyHostToDevice),
-           "set_scalar");
   return FREHG_GW_OK;
 }
 

@@ -255,9 +255,10 @@ struct PhaseTables {
   StepOut* outs_host = nullptr;  // pinned
   int cap = 0;                   // members the buffers hold (reused while n <= cap)
 };
-// (Re)builds the tables for the members `ds`, reusing the buffers while they fit.
+// (Re)builds the tables for the members `ds`, reusing the buffers while they
+// fit, uploaded on s, the stream that the batch's steps run on.
 cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>& ds,
-                               const std::vector<int>& mixed);
+                               const std::vector<int>& mixed, cudaStream_t s);
 void phase_tables_free(PhaseTables& t);
 void fill_step_args(const Device& D, bool mixed, double dtg, double co_max, double dq_grow,
                     double dq_shrink, double dt_min, double dt_max, StepArgs& a);
@@ -311,7 +312,8 @@ struct SolveGroup {
 size_t solve_group_bytes(const SolveClass& c, int n);
 // Builds a group over `ds` with `nb[i]` blocks each (all of solve kind c.kind,
 // member i in class variants[i]), its
-// tables placed in `mem` (solve_group_bytes of device memory the caller owns).
+// tables placed in `mem` (solve_group_bytes of device memory the caller owns)
+// and uploaded on `s`, the stream of its launches.
 // The launch takes min(sum nb, max_grid) co-resident blocks (max_grid at
 // least every nb[i]); each block takes the members' block slots from a queue,
 // so a member's slots go out together and the blocks of a converged member go
@@ -320,7 +322,8 @@ size_t solve_group_bytes(const SolveClass& c, int n);
 // re-ranked on the device before every launch.
 cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vector<Device*>& ds,
                               const std::vector<int>& variants, const std::vector<int>& nb,
-                              const std::vector<SolveParams>& p, int max_grid, void* mem);
+                              const std::vector<SolveParams>& p, int max_grid, void* mem,
+                              cudaStream_t s);
 // Zeroes the members' CG states and the slot queue and launches the group on `s`.
 cudaError_t solve_group_launch(const SolveGroup& g, cudaStream_t s);
 

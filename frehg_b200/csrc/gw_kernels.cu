@@ -2650,7 +2650,7 @@ void fill_step_args(const Device& D, bool mixed, double dtg, double co_max, doub
 }
 
 cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>& ds,
-                               const std::vector<int>& mixed) {
+                               const std::vector<int>& mixed, cudaStream_t s) {
   t.n = static_cast<int>(ds.size());
   cudaError_t e = cudaSuccess;
   if (t.n > t.cap) {
@@ -2681,11 +2681,15 @@ cudaError_t phase_tables_build(PhaseTables& t, const std::vector<const Device*>&
   t.grid_ghost = fg.back();
   t.grid_factor = ff.back();
   if (e == cudaSuccess)
-    e = cudaMemcpy(t.first_cells, fc.data(), sizeof(int) * fc.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(t.first_cells, fc.data(), sizeof(int) * fc.size(), cudaMemcpyHostToDevice,
+                        s);
   if (e == cudaSuccess)
-    e = cudaMemcpy(t.first_ghost, fg.data(), sizeof(int) * fg.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(t.first_ghost, fg.data(), sizeof(int) * fg.size(), cudaMemcpyHostToDevice,
+                        s);
   if (e == cudaSuccess)
-    e = cudaMemcpy(t.first_factor, ff.data(), sizeof(int) * ff.size(), cudaMemcpyHostToDevice);
+    e = cudaMemcpyAsync(t.first_factor, ff.data(), sizeof(int) * ff.size(), cudaMemcpyHostToDevice,
+                        s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e == cudaSuccess && t.walk_smem > 0)
     e = raise_smem_limit(reinterpret_cast<const void*>(k_walk_batch), t.walk_smem);
   return e;
