@@ -134,6 +134,19 @@ __device__ inline void cg64_cell_update(const Cg64Args& a, long long c, double a
   zz += z * z;
 }
 
+// After a solve that met a NaN or an overflow: the arrays of the assembly that
+// the solve wrote, cleared.  The assembly rewrites the interior's before every
+// solve, but never the ghost columns', where a scaled leg (0 / sqrt(NaN)) or
+// the one-barrier form's scratch would keep the NaN for every later step.
+__device__ inline void cg64_clear(const Cg64Args& a, long long t0, long long stride) {
+  for (long long c = t0; c < a.d.ncell; c += stride) {
+    a.gxp[c] = 0.0;
+    a.gyp[c] = 0.0;
+    a.gzp[c] = 0.0;
+    a.bw[c] = 0.0;
+  }
+}
+
 // The words of a thread's own cells held in shared memory, by what keeping
 // each saves in traffic: W of them, in this order.
 enum OwnWord { kOwnW = 0, kOwnY = 1, kOwnS = 2, kOwnGym = 3, kOwnGxm = 4, kOwnGx = 5, kOwnGy = 6 };
@@ -354,6 +367,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     fin(s.y, y.y, c + 1);
   }
   if (tail) fin(sa[ct], xa[ct], ct);
+  if (reason == -9) cg64_clear(a, t0, stride);
   if (bid == 0 && threadIdx.x == 0) {
     a.st->dp = dp;
     a.st->rnorm0 = rnorm0;
@@ -620,6 +634,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
     st2(a.x + c, s.x * y.x, s.y * y.y);
   }
   if (tail) a.x[ct] = ts * ty;
+  if (reason == -9) cg64_clear(a, t0, stride);
   if (bid == 0 && threadIdx.x == 0) {
     a.st->dp = dp;
     a.st->rnorm0 = rnorm0;

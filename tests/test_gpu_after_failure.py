@@ -1,0 +1,99 @@
+"""A solver whose step failed on bad data steps on as a new one does once it
+has good data again: nothing of the failed solve stays behind."""
+import numpy as np
+import pytest
+
+import cases
+from frehg_b200 import workloads
+from frehg_b200.batch import RichardsBatch
+from frehg_b200.gw import FatalError, RichardsSolver
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("h", "wc", "qx", "qy", "qz")
+
+
+def closed_cell(precision):
+    cfg = workloads.column_32x32x50(1, 1, 1, precision=precision)
+    cfg.boundary_conditions = []
+    return cfg
+
+
+def masked_box(precision):
+    cfg = cases.mixed_box(nx=9, ny=7, nz=13)
+    cfg.solver.precision = precision
+    return cfg
+
+
+def deep_box(precision):
+    """Past one block, odd depth; FP64 at 1e-12: two barriers an iteration."""
+    cfg = cases.mixed_box(nx=31, ny=29, nz=51)
+    cfg.solver.precision = precision
+    cfg.solver.rtol = 1e-12
+    return cfg
+
+
+def wide_box(precision):
+    """Past one block; FP64 at 1e-8: one barrier an iteration."""
+    cfg = cases.mixed_box(nx=31, ny=29, nz=51)
+    cfg.solver.precision = precision
+    return cfg
+
+
+BOXES = [closed_cell, masked_box, deep_box, wide_box]
+
+
+def bad_heads(head):
+    """A NaN in one cell; heads whose squares overflow FP32 and FP64."""
+    nan = head.copy()
+    nan[0, 0, 0] = np.nan
+    huge = np.where(np.arange(head.size).reshape(head.shape) % 2, 1e39, -1e39)
+    return {"nan": nan, "float": huge, "double": 1e200 * huge / 1e39}
+
+
+@pytest.mark.parametrize("box", BOXES)
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_line"])
+def test_step_after_failed_step(box, precision):
+    with RichardsSolver(box(precision)) as s, RichardsSolver(box(precision)) as new:
+        head, wc = s.head(), s.waterContent()
+        new.setState(head, wc)
+        new.step(0.0, 1.0)
+        want = {name: new.field(name) for name in FIELDS}
+        for what, bad in bad_heads(head).items():
+            s.setState(bad, wc)
+            try:
+                s.step(0.0, 1.0)
+            except FatalError:
+                pass
+            s.setState(head, wc)
+            s.step(0.0, 1.0)
+            for name in FIELDS:
+                np.testing.assert_array_equal(s.field(name), want[name], err_msg=f"{what} {name}")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batch_after_failed_step(precision):
+    def step(solvers, batch, heads, wcs):
+        for s, h, w in zip(solvers, heads, wcs):
+            s.setState(h, w)
+        for i in range(len(solvers)):
+            batch.set_dt(i, 1.0)
+        batch.step()
+
+    solvers = [RichardsSolver(box(precision)) for box in BOXES]
+    fresh = [RichardsSolver(box(precision)) for box in BOXES]
+    heads, wcs = [s.head() for s in solvers], [s.waterContent() for s in solvers]
+    with RichardsBatch(solvers) as b, RichardsBatch(fresh) as f:
+        step(fresh, f, heads, wcs)
+        for what in ("nan", "float", "double"):
+            try:
+                step(solvers, b, [bad_heads(h)[what] for h in heads], wcs)
+            except FatalError:
+                pass
+            step(solvers, b, heads, wcs)
+            for m, (s, n) in enumerate(zip(solvers, fresh)):
+                for name in FIELDS:
+                    np.testing.assert_array_equal(s.field(name), n.field(name),
+                                                  err_msg=f"{what} {m} {name}")
+    for s in solvers + fresh:
+        s.close()
