@@ -204,13 +204,13 @@ cudaError_t launch_cg_line64(Device& D, double atol, int maxit, double outer_rto
 cudaError_t raise_smem_limit(const void* kernel, size_t bytes);
 
 // ---------------------------------------------------------------- small domains
-// A groundwater-only domain up to kSmallCells cells runs the phases before
-// and after its solve as one cooperative launch each (k_small_pre,
-// k_small_post); the step record lands in D.out_host.  Above, the separate
-// launches' own occupancies win: whole steps, one launch a phase (with its
-// timing events, some 15 us) against two, FP64: 32x32x50 208 -> 153 us,
-// 56x56x80 279 -> 227, 64x64x128 377 -> 345, 80x80x128 482 -> 475,
-// 100x100x100 568 -> 557.
+// A groundwater-only domain up to kSmallCells cells (whose columns take the
+// warp walk) runs the phases before and after its solve as one cooperative
+// launch each (k_small_pre, k_small_post); the step record lands in
+// D.out_host.  Above, the separate launches' own occupancies win: whole steps,
+// one launch a phase (with its timing events, some 15 us) against two, FP64:
+// 32x32x50 208 -> 153 us, 56x56x80 279 -> 227, 64x64x128 377 -> 345, 80x80x128
+// 482 -> 475, 100x100x100 568 -> 557.
 constexpr long long kSmallCells = 600000;
 constexpr size_t kSmallSyncWords = 64;
 bool small_domain(const Device& D);

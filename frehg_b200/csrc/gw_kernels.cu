@@ -2340,16 +2340,12 @@ __global__ void __launch_bounds__(kBlock, 2) k_small_post(SmallArgs s) {
   update_wc_body<false>(a.d, a.f, a.hp, a.hn, a.wcn, a.qx, a.qy, a.qzf, dtgp, a.wcu, a.satf,
                         a.colflag, a.partial + kPSs * G, bid, G);
   if (!barrier()) return;
-  classify_body<false>(a.d, a.f, a.kx, a.ky, a.kzf, a.wcu, a.hp, a.satf, a.wc_out, a.h_out,
-                       a.warp_walk ? nullptr : a.room, a.sup, a.sdn, a.colflag, a.partial + kPAdj * G, a.partial + kPDrop * G, bid,
+  classify_body<false>(a.d, a.f, a.kx, a.ky, a.kzf, a.wcu, a.hp, a.satf, a.wc_out, a.h_out, nullptr,
+                       a.sup, a.sdn, a.colflag, a.partial + kPAdj * G, a.partial + kPDrop * G, bid,
                        G);
   if (!barrier()) return;
-  if (a.warp_walk)
-    walk_body<false>(a.d, a.f, a.wc_out, a.sup, a.sdn, a.qzf, a.colflag, dtgp, a.partial, G,
-                     nullptr, nullptr, bid, G);
-  else
-    walk_thread_body<false>(a.d, a.f, a.wc_out, a.room, a.sup, a.sdn, a.qzf, a.colflag, dtgp,
-                            a.partial, G, nullptr, nullptr, bid, G);
+  walk_body<false>(a.d, a.f, a.wc_out, a.sup, a.sdn, a.qzf, a.colflag, dtgp, a.partial, G, nullptr,
+                   nullptr, bid, G);
   if (!barrier()) return;
   finalize_body(a.d, a.f, a.wc_out, a.vloss, a.qx, a.qy, a.qzf, dtgp, a.co_max, a.partial, G, bid,
                 G);
@@ -2755,8 +2751,11 @@ int small_grid(const Device& D) {
 
 }  // namespace
 
+// (A column of the thread walk is one thread's work, up to seconds for
+// thousands of cells, at whose end the other blocks would wait in a barrier
+// that gives up: it keeps its own launch.)
 bool small_domain(const Device& D) {
-  return D.d.ncell <= kSmallCells && !D.f.cpl && !D.f.baro && !D.win_x;
+  return D.d.ncell <= kSmallCells && !D.f.cpl && !D.f.baro && !D.win_x && warp_walk(D);
 }
 
 cudaError_t launch_small_pre(Device& D, bool mixed, bool warm, double dtg, const double* hprev,
@@ -2789,7 +2788,7 @@ cudaError_t launch_small_post(Device& D, double co_max, double dq_grow, double d
   s.arrived = D.small_sync + 32;  // a line of its own
   s.base = D.small_base[1];
   s.host = D.out_host;
-  const size_t smem = s.a.warp_walk ? kWalkWarps * walk_warp_bytes(D.d.nz) : 0;
+  const size_t smem = kWalkWarps * walk_warp_bytes(D.d.nz);
   cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(k_small_post), smem);
   if (e != cudaSuccess) return e;
   void* args[] = {&s};
