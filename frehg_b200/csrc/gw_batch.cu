@@ -173,15 +173,6 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   std::vector<int> first(ds.size() + 1, 0);
   std::vector<CgState*> st(ds.size());
   std::vector<double*> parts(ds.size());
-  for (size_t i = 0; i < ds.size(); ++i) {
-    if (c.kind == 0) cg64_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
-    else mixed_fill_args(*ds[i], p[i], variants[i], tab.data() + i * ab);
-    first[i + 1] = first[i] + nb[i];
-    st[i] = &ds[i]->out->cg;
-    parts[i] = ds[i]->cgpart;
-  }
-  g.slots = first.back();
-  g.grid = std::min(g.slots, max_grid);
   auto r = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
   char* base = static_cast<char*>(mem);
   g.tab = base;
@@ -189,6 +180,16 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   g.states = reinterpret_cast<CgState**>(base + r(tab.size()) + r(first.size() * sizeof(int)));
   char* q = base + r(tab.size()) + r(first.size() * sizeof(int)) +
             r(st.size() * sizeof(CgState*));
+  for (size_t i = 0; i < ds.size(); ++i) {
+    const Peers peers{g.states, g.n};
+    if (c.kind == 0) cg64_fill_args(*ds[i], p[i], variants[i], peers, tab.data() + i * ab);
+    else mixed_fill_args(*ds[i], p[i], variants[i], peers, tab.data() + i * ab);
+    first[i + 1] = first[i] + nb[i];
+    st[i] = &ds[i]->out->cg;
+    parts[i] = ds[i]->cgpart;
+  }
+  g.slots = first.back();
+  g.grid = std::min(g.slots, max_grid);
   g.parts = reinterpret_cast<double**>(q);
   q += r(parts.size() * sizeof(double*));
   g.queue = reinterpret_cast<int*>(q);

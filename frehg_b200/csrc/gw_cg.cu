@@ -37,7 +37,7 @@
 // as the domain's size leaves room for).  512x512x128 (no room) 692 -> 571 us an
 // iteration, 131x113x127 (w) 48.2 -> 35.8, 64x64x128 (four) 12.7 -> 11.0.
 //
-// The grid barrier's wait is bounded: one that exceeds kSpinLimit polls sets
+// The grid barrier's wait is bounded: one that gives up (arrive_and_wait) sets
 // CgState::err, and every block leaves at its next barrier, so a launch that
 // lost co-residency ends with an error status instead of hanging.
 #include <algorithm>
@@ -65,6 +65,7 @@ struct Cg64Args {
   double rtol, atol;
   int maxit;
   int variant;  // batched solves: 1 = 16-byte pair accesses (nz even), 0 = separate loads
+  Peers peers;  // batched solves: the launch's members
 };
 
 // Up to this many pairs one block solves alone, without the grid barrier.
@@ -270,7 +271,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   }
   if (tail) cg64_cell_init(a, ct, rr, zz);
   double s2[2] = {zz, rr};
-  if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st)) return;
+  if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
   double dp = sqrt(s2[0]);
   double beta = s2[1];
   const double rnorm0 = dp;
@@ -307,7 +308,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       pw = cg64_phase_a<ALIGNED, W, false, false>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
     if (tail) cg64_cell_stencil(a, ct, i == 0, (i & 1) != 0, bc, al, al1, pold, pnew, pw);
     double s1[1] = {pw};
-    if (!grid_sum<kCgBlock>(s1, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(s1, a.part, bid, G, epoch, a.st, a.peers)) return;
     dpiold = dpi;
     dpi = s1[0];
     betaold = beta;
@@ -337,7 +338,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     if (tail) cg64_cell_update(a, ct, al, rr, zz);
     s2[0] = zz;
     s2[1] = rr;
-    if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
     dp = sqrt(s2[0]);
     test(dp);
     if (reason != 0) break;
@@ -533,7 +534,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
     zz += (ts * r) * (ts * r);
   }
   double v2[2] = {zz, rr};
-  if (!grid_sum<kCgBlock>(v2, a.part, bid, G, epoch, a.st)) return;
+  if (!grid_sum<kCgBlock>(v2, a.part, bid, G, epoch, a.st, a.peers)) return;
   double dp = sqrt(v2[0]), gamma = v2[1];
   const double rnorm0 = dp;
   const double ttol = fmax(a.rtol * rnorm0, a.atol);
@@ -578,7 +579,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
                                            nullptr, wb[0], nullptr, t0, stride, rr, rw, zz);
     if (tail) tail_cell(true, false, 0.0, 0.0, rb[0], nullptr, nullptr, nullptr, wb[0], nullptr);
     double v1[1] = {rw};
-    if (!grid_sum<kCgBlock>(v1, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(v1, a.part, bid, G, epoch, a.st, a.peers)) return;
     delta = v1[0];
   }
   double gold = 1.0, al = 1.0, dpi = 0.0, dpiold = 0.0;
@@ -614,7 +615,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
     if (tail)
       tail_cell(false, i == 0, al, be, rb[f], wb[f], sb[f], rb[1 - f], wb[1 - f], sb[1 - f]);
     double v3[3] = {zz, rr, rw};
-    if (!grid_sum<kCgBlock>(v3, a.part, bid, G, epoch, a.st)) return;
+    if (!grid_sum<kCgBlock>(v3, a.part, bid, G, epoch, a.st, a.peers)) return;
     dp = sqrt(v3[0]);
     test(dp);
     if (reason != 0) break;
@@ -787,9 +788,11 @@ cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool cle
 
 size_t cg64_args_bytes() { return sizeof(Cg64Args); }
 
-void cg64_fill_args(const Device& D, const SolveParams& p, int variant, void* dst) {
+void cg64_fill_args(const Device& D, const SolveParams& p, int variant, const Peers& peers,
+                    void* dst) {
   Cg64Args a = make_cg64_args(D, p.rtol, p.atol, p.maxit);
   a.variant = variant;
+  a.peers = peers;
   std::memcpy(dst, &a, sizeof(a));
 }
 

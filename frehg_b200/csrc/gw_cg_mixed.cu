@@ -156,9 +156,11 @@ int mixed_variant(const Device& D, bool tiled) { return tiled ? kLineDeep : line
 
 size_t mixed_args_bytes() { return sizeof(LineArgs<float>); }
 
-void mixed_fill_args(const Device& D, const SolveParams& p, int variant, void* dst) {
+void mixed_fill_args(const Device& D, const SolveParams& p, int variant, const Peers& peers,
+                     void* dst) {
   LineArgs<float> a = make_mixed_args(D, p.atol, p.maxit, p.outer_rtol, p.max_outer);
   a.variant = variant;
+  a.peers = peers;
   std::memcpy(dst, &a, sizeof(a));
 }
 

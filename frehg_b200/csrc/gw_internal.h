@@ -25,6 +25,13 @@ struct CgState {
   unsigned arrived; // blocks counted in at the solve's barriers (coop::grid_sum)
 };
 
+// The domains of a batched solve launch, n of them (0: a domain alone), whose
+// arrivals a barrier's wait watches.
+struct Peers {
+  CgState* const* states = nullptr;
+  int n = 0;
+};
+
 // Step results assembled on the device by k_step_info.
 struct StepOut {
   double boundary_in, ss_storage, realloc_adjust, realloc_dropped, vloss;
@@ -329,11 +336,13 @@ cudaError_t solve_group_launch(const SolveGroup& g, cudaStream_t s);
 
 // Per-kind pieces of the batched solves (gw_cg.cu, gw_cg_mixed.cu).
 size_t cg64_args_bytes();
-void cg64_fill_args(const Device& D, const SolveParams& p, int variant, void* dst);
+void cg64_fill_args(const Device& D, const SolveParams& p, int variant, const Peers& peers,
+                    void* dst);
 const void* cg64_batch_kernel();
 int mixed_variant(const Device& D, bool tiled);
 size_t mixed_args_bytes();
-void mixed_fill_args(const Device& D, const SolveParams& p, int variant, void* dst);
+void mixed_fill_args(const Device& D, const SolveParams& p, int variant, const Peers& peers,
+                     void* dst);
 const void* mixed_batch_kernel();
 
 }  // namespace fgw
