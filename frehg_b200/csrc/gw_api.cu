@@ -706,7 +706,12 @@ int finish_step(frehg_gw_handle* h, frehg_gw_step_info* info) {
   s.next_dt = o.next_dt;
   int status = FREHG_GW_OK;
   if (o.cg.err) {
-    status = fail(FREHG_GW_ECUDA, "predictor solve: grid barrier timed out");
+    // The flag goes now: k_small_pre's other blocks read it in their first
+    // barrier, unordered with its clearing there.
+    const cudaError_t e = cudaMemsetAsync(&D.out->cg, 0, sizeof(fgw::CgState), D.stream);
+    status = e == cudaSuccess
+                 ? fail(FREHG_GW_ECUDA, "predictor solve: grid barrier timed out")
+                 : cuda_fail(e, "predictor solve: grid barrier timed out; its reset");
   } else if (o.cg.reason < 0) {
     status = fail(FREHG_GW_ESOLVER, "predictor solve diverged after " + std::to_string(o.cg.its) +
                                         " iterations (KSP reason " +
@@ -786,7 +791,7 @@ int frehg_gw_step(frehg_gw_handle* h, double t, double dtg, frehg_gw_step_info* 
   }
   CUDA_TRY(cudaStreamSynchronize(D.stream), "step");
   CUDA_TRY(cudaGetLastError(), "step kernels");
-  if (small && D.out_host->cg.err) fgw::reset_small_sync(D);
+  if (small && D.out_host->cg.err) CUDA_TRY(fgw::reset_small_sync(D), "step barrier reset");
   if (prof) {
     for (int n = 0; n < 5; ++n) {
       float ms = 0.0f;
