@@ -573,7 +573,9 @@ struct LineSolve {
       // pass A wrote it, then the update of iteration `done` and, where
       // `done` is even, of the one before.
       pd.dset = done >= 1 || done == -2;
-      pd.p1 = (done & 1) ? a.v.p0 : a.v.p1;
+      // (Without an update, e1 = 0 multiplies the scaling: p0 and p1 may still
+      // hold an earlier solve's infinities.)
+      pd.p1 = done < 0 ? a.v.s : (done & 1) ? a.v.p0 : a.v.p1;
       pd.p2 = (done & 1) ? a.v.p1 : a.v.p0;
       pd.e1 = done >= 0 ? al : T(0);
       pd.e2 = (done >= 2 && !(done & 1)) ? al1 : T(0);

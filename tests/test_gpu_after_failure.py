@@ -71,6 +71,29 @@ def test_step_after_failed_step(box, precision):
                 np.testing.assert_array_equal(s.field(name), want[name], err_msg=f"{what} {name}")
 
 
+@pytest.mark.parametrize("precision", ["mixed", "fp64_line"])
+def test_exact_start_after_overflow(precision):
+    """At rest (head 0 everywhere, no boundary) the first residual is exactly 0
+    and the inner solve ends before it has a direction: no earlier step's may be
+    added.  Heads over the whole range in which some FP32 value of an iteration
+    overflows (factors of 1.5 apart; a product exceeds its factors by 2)."""
+    cfg = workloads.column_32x32x50(6, 5, 1, precision=precision)
+    cfg.boundary_conditions = []
+    rest = np.zeros((5, 6, 1))
+    full = np.full((5, 6, 1), 0.40)
+    sign = np.where(np.arange(30).reshape(5, 6, 1) % 2, 1.0, -1.0)
+    with RichardsSolver(cfg) as s:
+        for scale in 1e30 * 1.5 ** np.arange(100):
+            s.setState(scale * sign, full)
+            try:
+                s.step(0.0, 600.0)
+            except FatalError:
+                pass
+            s.setState(rest, full)
+            s.step(0.0, 600.0)
+            np.testing.assert_array_equal(s.head(), rest, err_msg=str(scale))
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 def test_batch_after_failed_step(precision):
     def step(solvers, batch, heads, wcs):
