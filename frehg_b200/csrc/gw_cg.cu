@@ -6,7 +6,8 @@
 // p = z + (beta / beta_old) p, alpha = beta / p'Ap, convergence on the
 // preconditioned norm ||z|| <= max(rtol ||D^-1 b||, atol), divergence at
 // 1e5 ||D^-1 b||, non-finite norms, indefinite matrix / preconditioner and
-// max_iterations.
+// max_iterations.  (A diagonal entry that is not positive, which no physical
+// data gives, ends as a non-finite norm.)
 //
 // The recurrences run on the system scaled to a unit diagonal: with
 // S = D^(-1/2), Jacobi-preconditioned CG on A x = b is plain CG on
@@ -285,7 +286,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   test(dp);
   double betaold = 1.0, dpi = 0.0, dpiold = 0.0;
   double al = 0.0, al1 = 0.0;  // a of the last two iterations
-  int i = 0, done = -1;        // done: the last iteration whose a is known
+  int i = 0, done = -1;        // done: the last iteration with an update pending
   while (reason == 0) {
     its = i + 1;
     if (beta == 0.0) {
@@ -313,6 +314,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     dpi = s1[0];
     betaold = beta;
     if (dpi == 0.0 || (i > 0 && sgn(dpi) * sgn(dpiold) < 0)) {
+      if (i & 1) done = -1;  // this iteration's phase A applied every update
       reason = -10;
       break;
     }

@@ -71,6 +71,28 @@ def test_step_after_failed_step(box, precision):
                 np.testing.assert_array_equal(s.field(name), want[name], err_msg=f"{what} {name}")
 
 
+# A lateral conductivity below zero makes the matrix indefinite under a positive
+# diagonal.  The iterations at which the curvature changes sign, even and odd.
+@pytest.mark.parametrize("ks,iterations", [(-1.2e-4, 8), (-1.3e-4, 7), (-1.4e-4, 6), (-1.5e-4, 5),
+                                           (-1.8e-4, 4), (-2.0e-4, 3)])
+def test_iterate_of_an_indefinite_solve(ks, iterations):
+    """The two forms of the FP64 solve end at the same iterate: the fluxes, which
+    are taken from it, agree to the parity bar."""
+    flux = {}
+    for rtol in (1e-10, 1e-11):  # one barrier an iteration, two
+        cfg = workloads.column_32x32x50(24, 20, 18)
+        cfg.soil_types[0].ksx = cfg.soil_types[0].ksy = ks
+        cfg.solver.rtol, cfg.solver.atol = rtol, 1e-300
+        cfg.initial.value = -1.0 - np.random.default_rng(3).random((20, 24, 18))
+        with RichardsSolver(cfg) as s:
+            with pytest.raises(FatalError) as e:
+                s.step(0.0, 100.0)
+            assert f"after {iterations} iterations (KSP reason -10)" in str(e.value)
+            flux[rtol] = [s.field(name) for name in ("qx", "qy", "qz")]
+    for a, b in zip(flux[1e-10], flux[1e-11]):
+        assert np.max(np.abs(a - b)) <= 1e-9 * np.max(np.abs(a))
+
+
 @pytest.mark.parametrize("precision", ["mixed", "fp64_line"])
 def test_exact_start_after_overflow(precision):
     """At rest (head 0 everywhere, no boundary) the first residual is exactly 0
