@@ -85,6 +85,14 @@ cudaError_t dalloc_margin(fgw::Device& D, T** p, long long ncell, long long marg
 constexpr int kFetchThreads = 4;
 constexpr size_t kFetchChunk = 2u << 20;
 constexpr size_t kFetchDirect = 8u << 20;  // smaller reads: one plain copy
+// Up to this size behind the packing with one wait for both (a wait of its own
+// for the packing was 5 us of an 8x6x20 read's 28, 8 of a 32x32x50 one's 59);
+// larger ones, 64x64x128 say, are slower as a stream's copy (300 against 289).
+constexpr size_t kFetchOrdered = 1u << 20;
+// Fields up to this size, halo and all, come over whole and are picked apart
+// here: no kernel (1x1x1 17 us against 22; 8x6x20, 13 KB, 21.5 against 23;
+// 8x8x32, 26 KB, 24.4 against 23.7).
+constexpr size_t kFetchWhole = 16u << 10;
 
 class FetchStaging {
  public:
@@ -159,11 +167,17 @@ cudaError_t fetch_range(int device, char* dst, const char* src, size_t lo, size_
   return e;
 }
 
-// Device to host, large copies by kFetchThreads threads at once (the host
-// side, first touches of the caller's pages above all, is what a large read
-// spends its time on).  The source must be complete.
-cudaError_t fetch(int device, double* dst, const double* src, size_t n) {
+// Device to host behind what s_src still has to do, large copies by
+// kFetchThreads threads at once (the host side, first touches of the caller's
+// pages above all, is what a large read spends its time on).
+cudaError_t fetch(int device, double* dst, const double* src, size_t n, cudaStream_t s_src) {
   const size_t bytes = n * sizeof(double);
+  if (bytes <= kFetchOrdered) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s_src);
+    return e == cudaSuccess ? cudaStreamSynchronize(s_src) : e;
+  }
+  const cudaError_t ready = cudaStreamSynchronize(s_src);
+  if (ready != cudaSuccess) return ready;
   char* const stage = bytes > kFetchDirect ? g_fetch.take() : nullptr;
   if (!stage) return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
   char* const d = reinterpret_cast<char*>(dst);
@@ -902,23 +916,24 @@ int frehg_gw_get_field(frehg_gw_handle* h, int field, double* out) {
   }
   // The owned part is packed on the device into a solve vector (scratch
   // between steps) and read back as one run.  A z-face field of a very flat
-  // domain can exceed it and is read whole.
+  // domain can exceed it and is read whole, as a small field is.
   const size_t count = frehg_gw_field_size(h, field);
-  if (count <= static_cast<size_t>(d.ncell)) {
+  const size_t nzf = static_cast<size_t>(kind == 3 ? d.nz + 1 : d.nz), all = d.ncol * nzf;
+  if (all * sizeof(double) > kFetchWhole && count <= static_cast<size_t>(d.ncell)) {
     fgw::launch_pack(D, src, kind, D.w);
     CUDA_TRY(cudaGetLastError(), "get_field");
-    CUDA_TRY(cudaStreamSynchronize(D.stream), "get_field");
-    CUDA_TRY(fetch(h->device, out, D.w, count), "get_field");
+    CUDA_TRY(fetch(h->device, out, D.w, count, D.stream), "get_field");
     return FREHG_GW_OK;
   }
-  std::vector<double> full(static_cast<size_t>(d.ncol) * (d.nz + 1));
+  std::vector<double> full(all);
   CUDA_TRY(cudaStreamSynchronize(D.stream), "get_field");
-  CUDA_TRY(cudaMemcpy(full.data(), src, full.size() * sizeof(double), cudaMemcpyDeviceToHost),
+  CUDA_TRY(cudaMemcpy(full.data(), src, all * sizeof(double), cudaMemcpyDeviceToHost),
            "get_field");
-  size_t q = 0;
-  for (int j = 1; j <= d.ny; ++j)
-    for (int i = 1; i <= d.nx; ++i)
-      for (int k = 0; k <= d.nz; ++k) out[q++] = full[fgw::fidx(d, j, i, k)];
+  const int j0 = kind == 2 ? 0 : 1, i0 = kind == 1 ? 0 : 1;
+  const size_t row = static_cast<size_t>(d.nx + 1 - i0) * nzf;
+  for (int j = j0; j <= d.ny; ++j)
+    std::memcpy(out + (j - j0) * row, full.data() + fgw::col2(d, j, i0) * nzf,
+                row * sizeof(double));
   return FREHG_GW_OK;
 }
 
