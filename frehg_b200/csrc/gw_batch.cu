@@ -52,23 +52,16 @@ namespace fgw {
 
 namespace {
 
-// Before a group's solve launch, block 0: ranks the members by estimated
+// Before a group's solve launch, one block: ranks the members by estimated
 // work, nb (iterations of the previous solve + 4), largest first, ties by
 // table index (up to kRankMax members; beyond, table order), writes the queue
 // order and its slot offsets, then zeroes the members' CG states and the
-// slot counter; the other blocks zero the members' reduction slots.  The order only decides which member's slots go out first;
+// slot counter.  The order only decides which member's slots go out first;
 // a member's arithmetic depends on its own block count alone.
 constexpr int kRankMax = 1024;
 
-__global__ void k_queue_setup(CgState** st, double* const* __restrict__ parts,
-                              const int* __restrict__ first, int n, int* queue, int* order,
-                              int* ofirst) {
-  if (blockIdx.x > 0) {
-    for (int i = blockIdx.x - 1; i < n; i += gridDim.x - 1)
-      for (int w = threadIdx.x; w < coop::kRedSlots * (first[i + 1] - first[i]); w += blockDim.x)
-        parts[i][w] = 0.0;
-    return;
-  }
+__global__ void k_queue_setup(CgState** st, const int* __restrict__ first, int n, int* queue,
+                              int* order, int* ofirst) {
   __shared__ int part[256];
   const int t = threadIdx.x;
   if (n <= kRankMax) {
@@ -159,7 +152,7 @@ int solve_max_blocks(const Device& D, const SolveClass& c) {
 size_t solve_group_bytes(const SolveClass& c, int n) {
   auto r = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
   return r(args_bytes(c) * n) + r(sizeof(int) * (n + 1)) + r(sizeof(CgState*) * n) +
-         r(sizeof(double*) * n) + r(sizeof(int)) + r(sizeof(int) * n) + r(sizeof(int) * (n + 1));
+         r(sizeof(int)) + r(sizeof(int) * n) + r(sizeof(int) * (n + 1));
 }
 
 cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vector<Device*>& ds,
@@ -172,7 +165,6 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   std::vector<unsigned char> tab(ab * ds.size());
   std::vector<int> first(ds.size() + 1, 0);
   std::vector<CgState*> st(ds.size());
-  std::vector<double*> parts(ds.size());
   auto r = [](size_t b) { return (b + 255) & ~static_cast<size_t>(255); };
   char* base = static_cast<char*>(mem);
   g.tab = base;
@@ -186,12 +178,9 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
     else mixed_fill_args(*ds[i], p[i], variants[i], peers, tab.data() + i * ab);
     first[i + 1] = first[i] + nb[i];
     st[i] = &ds[i]->out->cg;
-    parts[i] = ds[i]->cgpart;
   }
   g.slots = first.back();
   g.grid = std::min(g.slots, max_grid);
-  g.parts = reinterpret_cast<double**>(q);
-  q += r(parts.size() * sizeof(double*));
   g.queue = reinterpret_cast<int*>(q);
   g.order = reinterpret_cast<int*>(q + r(sizeof(int)));
   g.ofirst = reinterpret_cast<int*>(q + r(sizeof(int)) + r(sizeof(int) * ds.size()));
@@ -202,15 +191,12 @@ cudaError_t solve_group_build(SolveGroup& g, const SolveClass& c, const std::vec
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(g.states, st.data(), st.size() * sizeof(CgState*),
                         cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(g.parts, parts.data(), parts.size() * sizeof(double*),
-                        cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   return e;
 }
 
 cudaError_t solve_group_launch(const SolveGroup& g, cudaStream_t s) {
-  k_queue_setup<<<1 + std::min(g.n, 128), 256, 0, s>>>(g.states, g.parts, g.first, g.n, g.queue, g.order, g.ofirst);
+  k_queue_setup<<<1, 256, 0, s>>>(g.states, g.first, g.n, g.queue, g.order, g.ofirst);
   void* tab = g.tab;
   int* first = g.first;
   int n = g.n;

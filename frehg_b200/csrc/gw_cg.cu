@@ -61,7 +61,7 @@ struct Cg64Args {
   double *gxp, *gyp, *gzp;       // scaled in place
   double *x, *r, *z, *p0, *p1, *w;  // x holds y and z holds s until the end
   double* bw;                       // b's array, free once r is made
-  double* part;  // kRedSlots x G, zero before the launch
+  double* part;  // kRedSlots x G (read only behind the write of the same barrier)
   CgState* st;
   double rtol, atol;
   int maxit;

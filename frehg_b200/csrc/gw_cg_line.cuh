@@ -475,7 +475,6 @@ struct LineSolve {
         for (int u = 0; u < kPassB; ++u) {
           place(a, base + u * step, 0, p[u]);
           const long long c = p[u].cp + p[u].k0;
-          if (W > 0 && u > 0 && base + u * step >= ncols) break;  // no words past the last
           ld_own<kLineW>(own, m + u, wv + c, p[u].n, w[u]);
           ld_own<kLineR>(own, m + u, rv + c, p[u].n, r[u]);
           ld_own<kLineL>(own, m + u, lv + c, p[u].n, l[u]);

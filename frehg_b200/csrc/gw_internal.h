@@ -310,7 +310,6 @@ struct SolveGroup {
   void* tab = nullptr;           // device table of per-member kernel arguments
   int* first = nullptr;          // device block offsets, n + 1
   CgState** states = nullptr;    // device array of the members' CG states
-  double** parts = nullptr;      // device array of the members' reduction slots
   int* queue = nullptr;          // device counter of the slots handed out
   int* order = nullptr;          // device queue order of the members, n
   int* ofirst = nullptr;         // device slot offsets in queue order, n + 1
