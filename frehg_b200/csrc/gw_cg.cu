@@ -227,7 +227,8 @@ __device__ __forceinline__ double cg64_phase_a(const Cg64Args& a, double2* __res
 }
 
 // W words of every own cell in shared memory (own, `words` pairs apart).
-template <bool ALIGNED, int W>
+// WATCH: in a batched launch.
+template <bool ALIGNED, int W, bool WATCH = false>
 __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, const int G,
                                            double2* __restrict__ own, const int words) {
   const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy;
@@ -272,7 +273,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
   }
   if (tail) cg64_cell_init(a, ct, rr, zz);
   double s2[2] = {zz, rr};
-  if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
+  if (!grid_sum<kCgBlock, WATCH>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
   double dp = sqrt(s2[0]);
   double beta = s2[1];
   const double rnorm0 = dp;
@@ -309,12 +310,11 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       pw = cg64_phase_a<ALIGNED, W, false, false>(a, own, words, bc, al, al1, pold, pnew, t0, stride);
     if (tail) cg64_cell_stencil(a, ct, i == 0, (i & 1) != 0, bc, al, al1, pold, pnew, pw);
     double s1[1] = {pw};
-    if (!grid_sum<kCgBlock>(s1, a.part, bid, G, epoch, a.st, a.peers)) return;
+    if (!grid_sum<kCgBlock, WATCH>(s1, a.part, bid, G, epoch, a.st, a.peers)) return;
     dpiold = dpi;
     dpi = s1[0];
     betaold = beta;
     if (dpi == 0.0 || (i > 0 && sgn(dpi) * sgn(dpiold) < 0)) {
-      if (i & 1) done = -1;  // this iteration's phase A applied every update
       reason = -10;
       break;
     }
@@ -340,7 +340,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
     if (tail) cg64_cell_update(a, ct, al, rr, zz);
     s2[0] = zz;
     s2[1] = rr;
-    if (!grid_sum<kCgBlock>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
+    if (!grid_sum<kCgBlock, WATCH>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
     dp = sqrt(s2[0]);
     test(dp);
     if (reason != 0) break;
@@ -351,6 +351,7 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
       break;
     }
   }
+  if (reason == -10 && (its & 1) == 0) done = -1;  // the last phase A applied every update
   // x = S y with the pending updates: iteration `done`'s and, where its own
   // phase A did not apply the one before (even), that one's.
   const double e1 = done < 0 ? 0.0 : al, e2 = (done > 0 && !(done & 1)) ? al1 : 0.0;
@@ -536,7 +537,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
     zz += (ts * r) * (ts * r);
   }
   double v2[2] = {zz, rr};
-  if (!grid_sum<kCgBlock>(v2, a.part, bid, G, epoch, a.st, a.peers)) return;
+  if (!grid_sum<kCgBlock, false>(v2, a.part, bid, G, epoch, a.st, a.peers)) return;
   double dp = sqrt(v2[0]), gamma = v2[1];
   const double rnorm0 = dp;
   const double ttol = fmax(a.rtol * rnorm0, a.atol);
@@ -581,7 +582,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
                                            nullptr, wb[0], nullptr, t0, stride, rr, rw, zz);
     if (tail) tail_cell(true, false, 0.0, 0.0, rb[0], nullptr, nullptr, nullptr, wb[0], nullptr);
     double v1[1] = {rw};
-    if (!grid_sum<kCgBlock>(v1, a.part, bid, G, epoch, a.st, a.peers)) return;
+    if (!grid_sum<kCgBlock, false>(v1, a.part, bid, G, epoch, a.st, a.peers)) return;
     delta = v1[0];
   }
   double gold = 1.0, al = 1.0, dpi = 0.0, dpiold = 0.0;
@@ -617,7 +618,7 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
     if (tail)
       tail_cell(false, i == 0, al, be, rb[f], wb[f], sb[f], rb[1 - f], wb[1 - f], sb[1 - f]);
     double v3[3] = {zz, rr, rw};
-    if (!grid_sum<kCgBlock>(v3, a.part, bid, G, epoch, a.st, a.peers)) return;
+    if (!grid_sum<kCgBlock, false>(v3, a.part, bid, G, epoch, a.st, a.peers)) return;
     dp = sqrt(v3[0]);
     test(dp);
     if (reason != 0) break;
@@ -688,9 +689,9 @@ __global__ void __launch_bounds__(kCgBlock, 1)
     __syncthreads();
     if (slot >= first[n]) break;
     if (sa.variant) {
-      cg64v_body<true, 0>(sa, sb, sg, nullptr, 0);
+      cg64v_body<true, 0, true>(sa, sb, sg, nullptr, 0);
     } else {
-      cg64v_body<false, 0>(sa, sb, sg, nullptr, 0);
+      cg64v_body<false, 0, true>(sa, sb, sg, nullptr, 0);
     }
     __syncthreads();  // every thread is done with sa before the next slot's
   }

@@ -80,7 +80,8 @@ struct Pending {
 // order; W = 0 for chunked columns and domains too large.
 enum LineOwn { kLineW = 0, kLineR, kLineL, kLineGym, kLineGxm, kLineGx, kLineGy };
 
-template <typename T, int LPC, int E, bool DEEP, int W = 0>
+// WATCH: in a batched launch.
+template <typename T, int LPC, int E, bool DEEP, int W = 0, bool WATCH = false>
 struct LineSolve {
   static constexpr int kCols = 32 / LPC;
   static_assert(W == 0 || (E == 4 && !DEEP), "one quad a lane");
@@ -504,12 +505,12 @@ struct LineSolve {
       double s[3] = {0.0, 0.0, 0.0};
       if (o == 0) {
         outer<true>(a, own, pd, a.x0, a.x1, gwarp, nwarp, s[2], s[0], s[1]);
-        if (!grid_sum<kLineBlock>(s, a.part, bid, G, epoch, a.st, a.peers)) return;
+        if (!grid_sum<kLineBlock, WATCH>(s, a.part, bid, G, epoch, a.st, a.peers)) return;
         bnorm = sqrt(s[2]);
       } else {
         outer<false>(a, own, pd, cur ? a.x1 : a.x0, cur ? a.x0 : a.x1, gwarp, nwarp, s[2], s[0], s[1]);
         double s2[2] = {s[0], s[1]};
-        if (!grid_sum<kLineBlock>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
+        if (!grid_sum<kLineBlock, WATCH>(s2, a.part, bid, G, epoch, a.st, a.peers)) return;
         s[0] = s2[0];
         s[1] = s2[1];
         cur ^= 1;
@@ -552,7 +553,7 @@ struct LineSolve {
         else if (i == 1) s1[0] = pass_a<false, true, true>(a, own, false, bc, al, al1, pold, pnew, gwarp, nwarp);
         else if (i & 1) s1[0] = pass_a<false, true, false>(a, own, false, bc, al, al1, pold, pnew, gwarp, nwarp);
         else s1[0] = pass_a<false, false, false>(a, own, false, bc, al, al1, pold, pnew, gwarp, nwarp);
-        if (!grid_sum<kLineBlock>(s1, a.part, bid, G, epoch, a.st, a.peers)) return;
+        if (!grid_sum<kLineBlock, WATCH>(s1, a.part, bid, G, epoch, a.st, a.peers)) return;
         const double dpi = s1[0];
         if (!(dpi > 0.0)) {  // inner breakdown: keep d, the FP64 sweep decides
           if (i & 1) done = -2;  // this pass applied every update
@@ -564,7 +565,7 @@ struct LineSolve {
         done = i;
         ++total;
         double sb[1] = {pass_b(a, own, al, gwarp, nwarp)};
-        if (!grid_sum<kLineBlock>(sb, a.part, bid, G, epoch, a.st, a.peers)) return;
+        if (!grid_sum<kLineBlock, WATCH>(sb, a.part, bid, G, epoch, a.st, a.peers)) return;
         beta = sb[0];
         if (sqrt(beta) <= itol) break;
       }

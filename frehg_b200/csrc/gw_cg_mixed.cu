@@ -66,11 +66,11 @@ __global__ void __launch_bounds__(kLineBlock, 1)
     __syncthreads();
     if (slot >= first[n]) break;
     switch (sa.variant) {
-      case 0: LineSolve<float, 8, 4, false>::run(sa, sb, sg); break;
-      case 1: LineSolve<float, 16, 4, false>::run(sa, sb, sg); break;
-      case 2: LineSolve<float, 32, 4, false>::run(sa, sb, sg); break;
-      case 3: LineSolve<float, 32, 8, false>::run(sa, sb, sg); break;
-      default: LineSolve<float, 32, 8, true>::run(sa, sb, sg); break;
+      case 0: LineSolve<float, 8, 4, false, 0, true>::run(sa, sb, sg); break;
+      case 1: LineSolve<float, 16, 4, false, 0, true>::run(sa, sb, sg); break;
+      case 2: LineSolve<float, 32, 4, false, 0, true>::run(sa, sb, sg); break;
+      case 3: LineSolve<float, 32, 8, false, 0, true>::run(sa, sb, sg); break;
+      default: LineSolve<float, 32, 8, true, 0, true>::run(sa, sb, sg); break;
     }
     __syncthreads();  // every thread is done with sa before the next slot's
   }

@@ -12,13 +12,11 @@ namespace coop {
 // 64x64x128 mixed iteration takes 11.6 us against 14.0, FP64 12.7 against 13.1.
 constexpr int kCgBlock = 512;
 
-// A barrier's wait looks around every kSpinLook polls (1.6 s at 0.32 us a
-// poll) and gives up after kIdleLooks looks in a row (14 s) that saw nothing
-// move: no barrier arrival of any of the launch's domains.  In a batched
-// launch a domain's first blocks may wait for the rest of another domain's
-// whole solve, however long that is, before theirs are handed out.
-constexpr int kSpinLook = 5000000;
-constexpr int kIdleLooks = 9;
+// Polls after which a barrier's wait gives up: 14 s at 0.32 us a poll.  In a
+// batched launch a domain's first blocks may wait for the rest of another
+// domain's whole solve, however long that is, before theirs are handed out:
+// their limit starts over while any domain of the launch arrives at a barrier.
+constexpr long long kSpinLimit = 45000000LL;
 
 // Reduction slots of a solve on G blocks: two generations of kRedVals values,
 // one double per block each, at the head of a solve's `part` array.
@@ -58,27 +56,29 @@ __device__ inline double warp_sum(double v) {
 // Thread 0's part of a grid barrier: counts the block in on `arrived` and polls
 // it up to `want` (which may wrap: the two differ by less than 2^31), with the
 // block's writes released before and the others' acquired after.  Gives up
-// when nothing moves any more (kIdleLooks), or when another block has, by
-// setting *err.  peers: the launch's domains, none where it has only one.
+// past kSpinLimit polls, or when another block has, by setting *err.  With
+// WATCH the limit starts over when one of the launch's domains, peers, has
+// arrived somewhere since the last limit (the code of it cost a solve of one
+// domain registers: 131x113x127 35.5 -> 37.2 us an iteration).
+template <bool WATCH>
 __device__ inline int arrive_and_wait(unsigned* arrived, unsigned want, int* err,
                                       const Peers& peers) {
   fence_gpu();
   red_add(arrived, 1u);
-  int ok = 1, spins = 0, idle = 0;
+  int ok = 1;
+  long long spins = 0;
   unsigned seen = 0u;
   while (static_cast<int>(ld_relaxed_u32(arrived) - want) < 0) {
     ++spins;
-    if ((spins & 1023) == 0 && ld_relaxed_int(err) != 0) ok = 0;
-    if (spins == kSpinLook) {
+    if (WATCH && spins > kSpinLimit) {
       unsigned now = 0u;
       for (int i = 0; i < peers.n; ++i) now += ld_relaxed_u32(&peers.states[i]->arrived);
-      idle = now != seen ? 0 : idle + 1;
+      if (now != seen) spins = 0;
       seen = now;
-      spins = 0;
-      if (idle == kIdleLooks) ok = 0;
     }
-    if (!ok) {
+    if (spins > kSpinLimit || ((spins & 1023) == 0 && ld_relaxed_int(err) != 0)) {
       atomicExch(err, 1);
+      ok = 0;
       break;
     }
   }
@@ -90,7 +90,7 @@ __device__ inline int arrive_and_wait(unsigned* arrived, unsigned want, int* err
 __device__ inline bool grid_barrier(unsigned* arrived, unsigned want, int* err) {
   __shared__ int good;
   __syncthreads();
-  if (threadIdx.x == 0) good = arrive_and_wait(arrived, want, err, Peers{});
+  if (threadIdx.x == 0) good = arrive_and_wait<false>(arrived, want, err, Peers{});
   __syncthreads();
   return good != 0;
 }
@@ -125,10 +125,11 @@ __device__ inline double tree_sum(const double* w) {
 // sums themselves as their own flags saves a round trip, but every block then
 // polls G words: 22.5 us for the FP64 iteration (at 296 blocks).
 //
+// WATCH: a batched launch, whose domains are `peers`.
 // The wait is bounded (arrive_and_wait): when it gives up thread 0 sets
 // CgState::err and every block returns false here or at its next call, and
 // leaves the kernel.
-template <int BLOCK, int NV>
+template <int BLOCK, bool WATCH, int NV>
 __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const int bid,
                                          const int G, unsigned& epoch, CgState* st,
                                          const Peers& peers) {
@@ -154,7 +155,8 @@ __device__ __forceinline__ bool grid_sum(double (&v)[NV], double* slots, const i
       }
       __syncwarp();
       if (lane == 0) {
-        good = arrive_and_wait(&st->arrived, epoch * static_cast<unsigned>(G), &st->err, peers);
+        good = arrive_and_wait<WATCH>(&st->arrived, epoch * static_cast<unsigned>(G), &st->err,
+                                      peers);
       }
     }
     __syncthreads();
