@@ -382,28 +382,33 @@ __device__ __forceinline__ void cg64v_body(const Cg64Args& a, const int bid, con
 }
 
 // ---------------------------------------------------------------- one barrier an iteration
-// The same CG with one reduction an iteration (Chronopoulos and Gear, "s-step
-// iterative methods for symmetric linear systems", J. Comput. Appl. Math. 25,
-// 1989): with w = A r beside r, g = r'r and d = r'w,
-//   b = g / g_old,  a = g / (d - b g / a_old)        (p'Ap = d - b g / a_old)
-//   p = r + b p,  s = w + b s (= A p),  y += a p,  r -= a s,  w = A r,
-// so one pass and one barrier do what the stencil and the update pass do.  A
-// neighbour's new r is taken from its old r, w and s (three vectors read where
-// p needs two, all three in two buffers), which costs a large domain more
-// traffic than the barrier costs it; p and y must fit in shared memory beside
-// their thread.  The recurrence for s loses a little attainable accuracy, so
-// tight solves keep the two-barrier form (kOneBarrierRtol).
-// Per iteration, against the two-barrier form: 64x64x128 10.9 -> 9.8 us; a
-// 101x55x25 coupled pass 20.4 -> 16.3 ms.
-enum OneWord { kOneY = 0, kOneP, kOneS, kOneGym, kOneGxm, kOneGx, kOneGy };
+// The same CG with one reduction an iteration (G. Meurant, "Multitasking the
+// conjugate gradient method on the CRAY X-MP/48", Parallel Computing 5, 1987;
+// its stability in T. Chen and E. Carson, "Predict-and-recompute conjugate
+// gradient variants", SIAM J. Sci. Comput. 42, 2020): with w = A p,
+//   a = r'r / p'w,  r -= a w,  y += a p,  p = r + b p,  w = A p,
+// where b is predicted, ||r - a w||^2 = a^2 w'w - r'r, while a takes the r'r
+// that the pass summed.  So one pass and one barrier do what the stencil and
+// the update pass do.  A neighbour's new p is taken from its old r, w and p
+// (three vectors read where p alone needs two, all three in two buffers), which
+// costs a large domain more traffic than the barrier costs it; y must fit in
+// shared memory beside its thread.
+// r follows A p itself, so the residual stays as true as the two-barrier
+// form's.  (The form of Chronopoulos and Gear carries A p by a recurrence, whose
+// drift a nearly singular system magnifies: the mean head of a closed saturated
+// 40x40x40 box at specific storage 1e-9 moved by 5e-6 m in a step, 7e-8 here and
+// with two barriers.  An iteration of 64x64x128 took 9.8 us in it as well, one of
+// 48x48x100 7.0 against 7.5, of 97x61x75 12.1 against 11.9.)
+enum OneWord { kOneY = 0, kOneS, kOneGym, kOneGxm, kOneGx, kOneGy, kOneWords };
 
+// START: w = A r alone.  FIRST: the old p is the old r.
 template <bool ALIGNED, int W, bool START, bool FIRST>
 __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, const int words,
                                               double al, double be, const double* ro,
-                                              const double* wo, const double* so, double* rn,
-                                              double* wn, double* sn, long long t0,
-                                              long long stride, double& rr, double& rw,
-                                              double& zz) {
+                                              const double* wo, const double* po, double* rn,
+                                              double* wn, double* pn, long long t0,
+                                              long long stride, double& rr, double& zz, double& pw,
+                                              double& ww) {
   const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy;
   int o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
@@ -415,51 +420,37 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
       if (W > word) chip(word) = v;
       return v;
     };
-    // r - al (w + be s) of a pair (START: r; FIRST: r - al w)
+    // (r - al w) + be p of a pair (START: r)
     const auto next2 = [&](long long m) {
       double2 r = ld_far<ALIGNED>(ro + m);
       if (START) return r;
-      const double2 w = ld_far<ALIGNED>(wo + m);
-      if (FIRST) {
-        r.x -= al * w.x;
-        r.y -= al * w.y;
-      } else {
-        const double2 s = ld_far<ALIGNED>(so + m);
-        r.x -= al * (w.x + be * s.x);
-        r.y -= al * (w.y + be * s.y);
-      }
+      const double2 w = ld_far<ALIGNED>(wo + m), p = FIRST ? r : ld_far<ALIGNED>(po + m);
+      r.x = (r.x - al * w.x) + be * p.x;
+      r.y = (r.y - al * w.y) + be * p.y;
       return r;
     };
     const auto next1 = [&](long long m) {
-      return START ? ro[m] : FIRST ? ro[m] - al * wo[m] : ro[m] - al * (wo[m] + be * so[m]);
+      return START ? ro[m] : (ro[m] - al * wo[m]) + be * (FIRST ? ro[m] : po[m]);
     };
-    const double2 rym = next2(c - sy), rxm = next2(c - sx);
-    const double2 rxp = next2(c + sx), ryp = next2(c + sy);
-    const double rkm = next1(c - 1), rkp = next1(c + 2);
+    const double2 pym = next2(c - sy), pxm = next2(c - sx);
+    const double2 pxp = next2(c + sx), pyp = next2(c + sy);
+    const double pkm = next1(c - 1), pkp = next1(c + 2);
     const double2 gx = leg(kOneGx, a.gxp + c), gxm = leg(kOneGxm, a.gxp + c - sx);
     const double2 gy = leg(kOneGy, a.gyp + c), gym = leg(kOneGym, a.gyp + c - sy);
     const double2 gz = ld2(a.gzp + c);
     const double gzm = a.gzp[c - 1];
-    double2 r = ld2(ro + c);
+    double2 p = ld2(ro + c);
     if (!START) {
-      double2 s = ld2(wo + c), p = r;
-      double2 y = make_double2(0.0, 0.0);
-      if (!FIRST) {
-        const double2 sp = ld2(so + c), pp = chip(kOneP);
-        y = chip(kOneY);
-        s.x += be * sp.x;
-        s.y += be * sp.y;
-        p.x += be * pp.x;
-        p.y += be * pp.y;
-      }
-      y.x += al * p.x;
-      y.y += al * p.y;
-      chip(kOneP) = p;
+      const double2 w = ld2(wo + c), pp = FIRST ? p : ld2(po + c);
+      const double2 r = make_double2(p.x - al * w.x, p.y - al * w.y);
+      double2 y = FIRST ? make_double2(0.0, 0.0) : chip(kOneY);
+      y.x += al * pp.x;
+      y.y += al * pp.y;
       chip(kOneY) = y;
-      r.x -= al * s.x;
-      r.y -= al * s.y;
+      p.x = r.x + be * pp.x;
+      p.y = r.y + be * pp.y;
       st2(rn + c, r.x, r.y);
-      st2(sn + c, s.x, s.y);
+      st2(pn + c, p.x, p.y);
       const double2 S = W > kOneS ? chip(kOneS) : ld2(a.z + c);
       const double z0 = S.x * r.x, z1 = S.y * r.y;
       rr += r.x * r.x;
@@ -467,42 +458,44 @@ __device__ __forceinline__ void cg64_one_pass(const Cg64Args& a, double2* own, c
       zz += z0 * z0;
       zz += z1 * z1;
     }
-    double w0 = gym.x * rym.x;
-    w0 += gxm.x * rxm.x;
-    w0 += gzm * rkm;
-    w0 += r.x;
-    w0 += gz.x * r.y;
-    w0 += gx.x * rxp.x;
-    w0 += gy.x * ryp.x;
-    double w1 = gym.y * rym.y;
-    w1 += gxm.y * rxm.y;
-    w1 += gz.x * r.x;
-    w1 += r.y;
-    w1 += gz.y * rkp;
-    w1 += gx.y * rxp.y;
-    w1 += gy.y * ryp.y;
+    double w0 = gym.x * pym.x;
+    w0 += gxm.x * pxm.x;
+    w0 += gzm * pkm;
+    w0 += p.x;
+    w0 += gz.x * p.y;
+    w0 += gx.x * pxp.x;
+    w0 += gy.x * pyp.x;
+    double w1 = gym.y * pym.y;
+    w1 += gxm.y * pxm.y;
+    w1 += gz.x * p.x;
+    w1 += p.y;
+    w1 += gz.y * pkp;
+    w1 += gx.y * pxp.y;
+    w1 += gy.y * pyp.y;
     st2(wn + c, w0, w1);
-    rw += r.x * w0;
-    rw += r.y * w1;
+    pw += p.x * w0;
+    pw += p.y * w1;
+    ww += w0 * w0;
+    ww += w1 * w1;
   }
 }
 
 template <bool ALIGNED, int W>
 __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, const int G,
                                               double2* own, const int words) {
-  static_assert(W >= 2, "y and p stay with their thread");
+  static_assert(W >= 1, "y stays with its thread");
   const long long N2 = a.d.ncell / 2, sx = a.d.sx, sy = a.d.sy, ct = a.d.ncell - 1;
   // The last cell of an odd count, taken by the grid's last thread, with its
-  // own y, p and s in registers.
+  // own y and s in registers.
   const bool tail = !ALIGNED && (a.d.ncell & 1) && bid == G - 1 && threadIdx.x == blockDim.x - 1;
   const long long stride = static_cast<long long>(G) * blockDim.x;
   const long long t0 = bid * static_cast<long long>(blockDim.x) + threadIdx.x;
   double* const rb[2] = {a.r, a.p0};
   double* const wb[2] = {a.w, a.p1};
-  double* const sb[2] = {a.bw, a.x};
+  double* const pb[2] = {a.bw, a.x};
   unsigned epoch = 0;
 
-  double rr = 0.0, zz = 0.0, rw = 0.0, ty = 0.0, tp = 0.0, ts = 0.0;
+  double rr = 0.0, zz = 0.0, pw = 0.0, ww = 0.0, ty = 0.0, ts = 0.0;
   int o = threadIdx.x;
   for (long long q = t0; q < N2; q += stride, o += kCgBlock) {
     const long long c = 2 * q;
@@ -550,42 +543,42 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
   test(dp);
   // The tail cell's share of a pass, on the buffers the pairs use.
   const auto tail_cell = [&](bool start, bool first, double al, double be, const double* ro,
-                             const double* wo, const double* so, double* rn, double* wn,
-                             double* sn) {
+                             const double* wo, const double* po, double* rn, double* wn,
+                             double* pn) {
     const auto nx = [&](long long m) {
-      return start ? ro[m] : first ? ro[m] - al * wo[m] : ro[m] - al * (wo[m] + be * so[m]);
+      return start ? ro[m] : (ro[m] - al * wo[m]) + be * (first ? ro[m] : po[m]);
     };
-    double r = ro[ct];
+    double p = ro[ct];
     if (!start) {
-      const double s = first ? wo[ct] : wo[ct] + be * so[ct];
-      tp = first ? r : r + be * tp;
-      ty += al * tp;
-      r -= al * s;
+      const double pp = first ? p : po[ct], r = p - al * wo[ct];
+      ty += al * pp;
+      p = r + be * pp;
       rn[ct] = r;
-      sn[ct] = s;
+      pn[ct] = p;
       rr += r * r;
       zz += (ts * r) * (ts * r);
     }
     double wv = a.gyp[ct - sy] * nx(ct - sy);
     wv += a.gxp[ct - sx] * nx(ct - sx);
     wv += a.gzp[ct - 1] * nx(ct - 1);
-    wv += r;
+    wv += p;
     wv += a.gzp[ct] * nx(ct + 1);
     wv += a.gxp[ct] * nx(ct + sx);
     wv += a.gyp[ct] * nx(ct + sy);
     wn[ct] = wv;
-    rw += r * wv;
+    pw += p * wv;
+    ww += wv * wv;
   };
-  double delta = 0.0;
-  if (reason == 0) {  // w = A r
+  if (reason == 0) {  // p = r, w = A p
     cg64_one_pass<ALIGNED, W, true, false>(a, own, words, 0.0, 0.0, rb[0], nullptr, nullptr,
-                                           nullptr, wb[0], nullptr, t0, stride, rr, rw, zz);
+                                           nullptr, wb[0], nullptr, t0, stride, rr, zz, pw, ww);
     if (tail) tail_cell(true, false, 0.0, 0.0, rb[0], nullptr, nullptr, nullptr, wb[0], nullptr);
-    double v1[1] = {rw};
+    double v1[2] = {pw, ww};
     if (!grid_sum<kCgBlock, false>(v1, a.part, bid, G, epoch, a.st, a.peers)) return;
-    delta = v1[0];
+    pw = v1[0];
+    ww = v1[1];
   }
-  double gold = 1.0, al = 1.0, dpi = 0.0, dpiold = 0.0;
+  double dpi = 0.0, dpiold = 0.0;
   int i = 0;
   while (reason == 0) {
     its = i + 1;
@@ -593,37 +586,33 @@ __device__ __forceinline__ void cg64_one_body(const Cg64Args& a, const int bid, 
       reason = 3;
       break;
     }
-    if (i > 0 && gamma * gold < 0.0) {
-      reason = -8;
-      break;
-    }
-    const double be = (i == 0) ? 0.0 : gamma / gold;
     dpiold = dpi;
-    dpi = (i == 0) ? delta : delta - be * gamma / al;
+    dpi = pw;
     if (dpi == 0.0 || (i > 0 && sgn(dpi) * sgn(dpiold) < 0)) {
       reason = -10;
       break;
     }
-    al = gamma / dpi;
-    gold = gamma;
+    const double al = gamma / dpi;
+    const double be = fmax(al * al * ww - gamma, 0.0) / gamma;
     const int f = i & 1;
-    rr = rw = zz = 0.0;
+    rr = zz = pw = ww = 0.0;
     if (i == 0)
-      cg64_one_pass<ALIGNED, W, false, true>(a, own, words, al, be, rb[f], wb[f], sb[f], rb[1 - f],
-                                             wb[1 - f], sb[1 - f], t0, stride, rr, rw, zz);
+      cg64_one_pass<ALIGNED, W, false, true>(a, own, words, al, be, rb[f], wb[f], pb[f], rb[1 - f],
+                                             wb[1 - f], pb[1 - f], t0, stride, rr, zz, pw, ww);
     else
-      cg64_one_pass<ALIGNED, W, false, false>(a, own, words, al, be, rb[f], wb[f], sb[f],
-                                              rb[1 - f], wb[1 - f], sb[1 - f], t0, stride, rr, rw,
-                                              zz);
+      cg64_one_pass<ALIGNED, W, false, false>(a, own, words, al, be, rb[f], wb[f], pb[f],
+                                              rb[1 - f], wb[1 - f], pb[1 - f], t0, stride, rr, zz,
+                                              pw, ww);
     if (tail)
-      tail_cell(false, i == 0, al, be, rb[f], wb[f], sb[f], rb[1 - f], wb[1 - f], sb[1 - f]);
-    double v3[3] = {zz, rr, rw};
-    if (!grid_sum<kCgBlock, false>(v3, a.part, bid, G, epoch, a.st, a.peers)) return;
-    dp = sqrt(v3[0]);
+      tail_cell(false, i == 0, al, be, rb[f], wb[f], pb[f], rb[1 - f], wb[1 - f], pb[1 - f]);
+    double v4[4] = {zz, rr, pw, ww};
+    if (!grid_sum<kCgBlock, false>(v4, a.part, bid, G, epoch, a.st, a.peers)) return;
+    dp = sqrt(v4[0]);
     test(dp);
     if (reason != 0) break;
-    gamma = v3[1];
-    delta = v3[2];
+    gamma = v4[1];
+    pw = v4[2];
+    ww = v4[3];
     ++i;
     if (i >= a.maxit) {
       reason = -3;
@@ -748,10 +737,12 @@ int cg64_words(long long pairs) {
 }
 
 // Solves at least this loose, of at most this many pairs a thread on more than
-// one block, take one barrier an iteration; beyond, the third vector's traffic
-// outweighs the barrier (us an iteration, two barriers against one: 48x48x100
-// 8.6 / 6.9, 97x61x75 14.4 / 13.3, 80x80x128 with six pairs 13.4 / 12.8, 81x80x127
-// with six 18.4 / 18.8, 90x90x128 with eight 15.6 / 17.2).
+// one block, take one barrier an iteration (us an iteration, two barriers
+// against one: 32x32x50 7.2 / 5.7, 101x55x25 7.7 / 6.1, 48x48x100 8.7 / 7.5,
+// 64x64x128 11.0 / 9.8, 97x61x75 12.6 / 11.9, 80x83x103 with five pairs 14.6 /
+// 14.1).  Beyond, the third vector's traffic outweighs the barrier (81x80x127
+// with six 18.4 / 18.8, 90x90x128 with eight 15.6 / 17.2).  Tighter solves keep
+// two: the predicted b has an error of eps r'r / (the next r'r).
 constexpr double kOneBarrierRtol = 1.0e-10;
 constexpr long long kOneBarrierPairs = 5;
 
@@ -776,9 +767,9 @@ cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool cle
   const long long pairs = std::max<long long>(1, (D.d.ncell / 2 + threads - 1) / threads);
   const int w = cg64_words(pairs);
   int words = static_cast<int>(pairs * kCgBlock);
-  const size_t smem = w * words * sizeof(double2);
   const bool even = D.d.nz % 2 == 0, one = w >= 2 && pairs <= kOneBarrierPairs &&
                                          D.cg_grid > 1 && rtol >= kOneBarrierRtol;
+  const size_t smem = (one ? std::min(w, kOneWords) : w) * words * sizeof(double2);
   const Cg64Kernel k = one ? (even ? cg64_one_kernel<true>(w) : cg64_one_kernel<false>(w))
                            : (even ? cg64_kernel<true>(w) : cg64_kernel<false>(w));
   const void* kern = reinterpret_cast<const void*>(k);
