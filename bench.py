@@ -49,20 +49,19 @@ ALG_BYTES_MIXED_INNER = 54    # FP32 inner iteration: stencil pass 8.5 words (z,
                               # gx, gy, l in; p, w out; every second iteration d and
                               # the p before in, d out), update + line solve 5 words
                               # (r, w, l in; r, z out)
-ALG_BYTES_MIXED_FIRST = 12    # less in each inner solve's first iteration (p = z:
-                              # neither p_old nor d)
-ALG_BYTES_MIXED_SWEEP = 76    # FP64 outer residual sweep: x, b, 4 coefficients, d, l,
-                              # scale in; x, r, z out
-ALG_BYTES_MIXED_OUTER = 8     # per correction: its last update's p, read by the next
-                              # sweep, and the d reset
-ALG_BYTES_MIXED_INIT = 12     # b read for ||b||, d = 0 at entry (the assembly writes
-                              # the starting iterate x = h^n)
+ALG_BYTES_MIXED_FIRST = 12    # less in each inner solve's first two iterations (p = z: no
+                              # p_old; then d = its first update: neither d nor the p
+                              # before in)
+ALG_BYTES_MIXED_SWEEP = 72    # FP64 outer residual sweep: x, b, 4 coefficients, scale, l
+                              # in; r, z out; and x out, or on the first one gx, gy out
+ALG_BYTES_MIXED_OUTER = 10    # per correction, in the sweep behind it: d and the pending
+                              # updates' p (two of them after every other solve)
 ALG_BYTES_FIXED = 536         # FP64 step outside the solve
 METRIC = "cell-steps/s at 512x512x128"
 # DRAM bytes (read + write) per algorithmic byte of k_cg_mixed, from the ncu
 # capture summarised in profiles/ (256x256x128 slab, one steady-state launch);
 # scaled to the timed launches by their algorithmic bytes.
-MIXED_TRAFFIC_PER_ALG_BYTE = 1.020
+MIXED_TRAFFIC_PER_ALG_BYTE = 1.029
 # Bytes frehg_gw_step reads back per step: the device step record (nine FP64
 # audit and controller terms, the solver's exit state, the coupled-top books).
 STEP_RECORD_BYTES = 192
@@ -73,8 +72,7 @@ def mixed_alg_bytes(cells, inner, outer, launches):
     inner iterations and `outer` outer corrections in total."""
     sweeps = outer + launches
     return cells * (ALG_BYTES_MIXED_INNER * inner - ALG_BYTES_MIXED_FIRST * outer +
-                    ALG_BYTES_MIXED_SWEEP * sweeps + ALG_BYTES_MIXED_OUTER * outer +
-                    ALG_BYTES_MIXED_INIT * launches)
+                    ALG_BYTES_MIXED_SWEEP * sweeps + ALG_BYTES_MIXED_OUTER * outer)
 
 
 def parse():

@@ -87,7 +87,7 @@ constexpr size_t kFetchChunk = 2u << 20;
 constexpr size_t kFetchDirect = 8u << 20;  // smaller reads: one plain copy
 // Up to this size behind the packing with one wait for both (a wait of its own
 // for the packing was 5 us of an 8x6x20 read's 28, 8 of a 32x32x50 one's 59);
-// larger ones, 64x64x128 say, are slower as a stream's copy (300 against 289).
+// a larger one does not notice (64x64x128: 285 to 325 us either way).
 constexpr size_t kFetchOrdered = 1u << 20;
 // Fields up to this size, halo and all, come over whole and are picked apart
 // here: no kernel (1x1x1 17 us against 22; 8x6x20, 13 KB, 21.5 against 23;

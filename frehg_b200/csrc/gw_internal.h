@@ -231,8 +231,9 @@ cudaError_t reset_small_sync(Device& D);
 // ---------------------------------------------------------------- batched phases
 // One member's arguments for the batched non-solve phases: its geometry and
 // fields, the state buffers of its current parity, its dt and controller
-// constants, and its per-kernel block counts (the single-domain launch's, so
-// a member's arithmetic in a batch is the single-domain step's bit for bit).
+// constants, and its block count (its own size's alone, so its arithmetic is the
+// same in every batch; against the single-domain step, whose block counts and
+// FP64 solve form may differ, sums agree to rounding).
 // The host refreshes the records before every batched step.
 struct alignas(16) StepArgs {
   Dims d;
@@ -291,8 +292,8 @@ struct SolveParams {
   int maxit, max_outer;
 };
 
-// Kernel variant of a domain's solve: FP64 (kind 0; variant 1 = two cells a
-// thread, nz even) or mixed (kind 1; variant = line_variant, or kLineDeep).
+// Kernel variant of a domain's solve: FP64 (kind 0; variant 1 = nz even, whose
+// neighbours' pairs are aligned) or mixed (kind 1; variant = line_variant, or kLineDeep).
 struct SolveClass {
   int kind, variant;
   bool operator==(const SolveClass& o) const { return kind == o.kind && variant == o.variant; }

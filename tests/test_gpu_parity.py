@@ -138,8 +138,8 @@ def test_slab_crop_64x64x128_parity():
 
 
 def test_deep_columns_parity():
-    # 190 cells: the deepest column whose warp walk needs more than the
-    # default 48 KB of shared memory per block; 257: the per-thread walk.
+    # Warp walks of 190 cells, which need more than the default 48 KB of shared
+    # memory per block, and of 257.
     compare(workloads.column_32x32x50(nx=3, ny=2, nz=190), 3)
     compare(workloads.column_32x32x50(nx=2, ny=2, nz=257), 2)
 

@@ -54,8 +54,8 @@ def compare(nx, ny, nz, precision, rtol):
         o.close()
 
 
-# 1, 33, 65, 129, 257: the first depth of each column variant; 32, 64, 128, 256:
-# the last; 4096 is the mixed form's deepest; others leave a padded quad.
+# 1, 33, 65, 129: the first depth of each column variant (257 below); 32, 64,
+# 128, 256: the last; others leave a padded quad.
 @pytest.mark.parametrize("nz", [1, 3, 32, 33, 64, 65, 127, 128, 129, 256])
 @pytest.mark.parametrize("precision", ["mixed", "fp64_line"])
 def test_column_depths(nz, precision):
@@ -74,8 +74,8 @@ def test_column_counts(nx, ny, precision):
     compare(nx, ny, 20, precision, 1e-12)
 
 
-# Odd and even cell counts; one block; seven, four and two words in shared
-# memory; one barrier (1e-10) and two (1e-12).
+# Odd and even cell counts; one block, and one to three pairs a thread on more
+# (seven or four words in shared memory); one barrier (1e-10) and two (1e-12).
 @pytest.mark.parametrize("shape", [(1, 1, 1), (1, 1, 5), (4, 3, 7), (13, 11, 9), (31, 29, 51),
                                    (64, 48, 63), (80, 50, 100)])
 @pytest.mark.parametrize("rtol", [1e-10, 1e-12])
