@@ -769,7 +769,7 @@ cudaError_t launch_cg64(Device& D, double rtol, double atol, int maxit, bool cle
   int words = static_cast<int>(pairs * kCgBlock);
   const bool even = D.d.nz % 2 == 0, one = w >= 2 && pairs <= kOneBarrierPairs &&
                                          D.cg_grid > 1 && rtol >= kOneBarrierRtol;
-  const size_t smem = (one ? std::min(w, kOneWords) : w) * words * sizeof(double2);
+  const size_t smem = (one ? std::min<int>(w, kOneWords) : w) * words * sizeof(double2);
   const Cg64Kernel k = one ? (even ? cg64_one_kernel<true>(w) : cg64_one_kernel<false>(w))
                            : (even ? cg64_kernel<true>(w) : cg64_kernel<false>(w));
   const void* kern = reinterpret_cast<const void*>(k);
