@@ -721,8 +721,10 @@ int finish_step(frehg_gw_handle* h, frehg_gw_step_info* info) {
   int status = FREHG_GW_OK;
   if (o.cg.err) {
     // The flag goes now: k_small_pre's other blocks read it in their first
-    // barrier, unordered with its clearing there.
-    const cudaError_t e = cudaMemsetAsync(&D.out->cg, 0, sizeof(fgw::CgState), D.stream);
+    // barrier, unordered with its clearing there.  (Waited for: the next step
+    // may be a batch's, on its own stream.)
+    cudaError_t e = cudaMemsetAsync(&D.out->cg, 0, sizeof(fgw::CgState), D.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(D.stream);
     status = e == cudaSuccess
                  ? fail(FREHG_GW_ECUDA, "predictor solve: grid barrier timed out")
                  : cuda_fail(e, "predictor solve: grid barrier timed out; its reset");
