@@ -54,12 +54,6 @@ __device__ inline double ghost_head_at(const Dims& d, const Fields& f, int code,
 struct SumOp {
   __device__ double operator()(double a, double b) const { return a + b; }
 };
-struct MaxOp {
-  __device__ double operator()(double a, double b) const { return b > a ? b : a; }
-};
-struct MinOp {
-  __device__ double operator()(double a, double b) const { return b < a ? b : a; }
-};
 
 // Block-wide reduction in a fixed order; the result is valid in thread 0.
 template <class Op>
